@@ -71,7 +71,7 @@ int compress_t(const gpz_params *p, const void *d_x, const void *d_y, const void
   const bool strict = (p->flags & GPZ_FLAG_STRICT_BOUND) != 0;
   const double *eb_dev = strict ? &ctl->strict_eb : nullptr;
   if (strict)
-    strict_bound_kernel<T><<<num_sms() * 4, 256, 0, st>>>(x, y, p->dim == 3 ? z : y, p->n, p->dim, eb, ctl);
+    strict_bound_kernel<T><<<num_sms() * 6, 256, 0, st>>>(x, y, p->dim == 3 ? z : y, p->n, p->dim, eb, ctl);
   if (p->flags & GPZ_FLAG_SEG_FIXED) {
     if (p->seg_size == 0) return GPZ_EINVAL;
     set_seg_kernel<<<1, 1, 0, st>>>(ctl, p->seg_size);
@@ -328,7 +328,9 @@ int gpz_rel_to_abs(uint32_t float_bits, uint32_t dim, uint64_t n, const void *d_
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Control *ctl = static_cast<Control *>(d_scratch);
   if (cudaMemsetAsync(d_scratch, 0, kCtlBytes, st) != cudaSuccess) return GPZ_ECUDA;
-  const int grid = num_sms() * 4;
+  // enough blocks for the loads in flight, no more than the work fills
+  const uint64_t per_block = 256ull * kFoldUnroll * (float_bits == 32 ? 4 : 2);
+  const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * 6, (n + per_block - 1) / per_block));
   if (float_bits == 32)
     rel_to_abs_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float *>(d_x), static_cast<const float *>(d_y),
                                                    static_cast<const float *>(dim == 3 ? d_z : d_y), n, dim,
