@@ -5,9 +5,9 @@
 // src/CompressorManager.cpp:12-16), so a workload of many small snapshots is
 // dominated by per-call launches, syncs and an almost idle GPU.  Here every
 // snapshot keeps its own stream, control block and look-back words; the
-// groups of 8 chunks of all snapshots of a class form one global work list
-// (snapshot after snapshot, so each snapshot's groups are claimed in order),
-// and one persistent kernel per class claims them.  A snapshot's stream is
+// chunks of all snapshots of a class form one global work list (snapshot
+// after snapshot, so each snapshot's chunks are claimed in order), and one
+// persistent kernel per class claims them.  A snapshot's stream is
 // byte-identical to the one gpz_compress writes for it: the per-chunk
 // encoder, the placement and the header/meta writes are the same code.
 #pragma once
@@ -21,124 +21,135 @@ namespace gpzb {
 constexpr uint32_t kBatchSegFixed = 1u;  // the segment size is given (no sampling)
 constexpr uint32_t kBatchSafe31 = 2u;    // GPZ_FLAG_SAFE31 rules for the automatic segment size
 constexpr uint32_t kBatchRelDev = 4u;    // absolute bound computed on the device from rel_eb
-constexpr int kBatchLocalBits = 40;      // map entry: item << 40 | group within the item
+constexpr uint32_t kBatchRelMode = 8u;   // the automatic segment size follows the relative-bound rules
+constexpr int kBatchLocalBits = 40;      // decompress map entry: item << 40 | chunk within the item
 
 // One snapshot of a batch.  `a` is what the single-stream kernel gets as its
 // parameter; a.eb is rewritten on the device when kBatchRelDev is set.
 template <typename T>
 struct BItem {
   CArgs<T> a;
-  Control *rctl;     // control block of the device rel->abs reduction
+  unsigned long long start;  // first chunk of the snapshot in the class's work list
   T rel_eb;
+  uint32_t seg;      // segment size resolved by the sampling kernel (0: it failed)
   uint32_t seg_in;
-  int32_t rel_mode;
   uint32_t flags;
 };
 
 // computeSegSize for every snapshot of the class (blockIdx.y = snapshot, 128
 // blocks each), or the given segment size.
 template <typename T>
-__global__ void __launch_bounds__(256) batch_sample_kernel(const BItem<T> *items) {
-  const BItem<T> &it = items[blockIdx.y];
+__global__ void __launch_bounds__(256) batch_sample_kernel(BItem<T> *items) {
+  BItem<T> &it = items[blockIdx.y];
   if (it.flags & kBatchSegFixed) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       it.a.ctl->seg = it.seg_in;
       it.a.ctl->adjusted = 0;
+      it.seg = it.seg_in;
     }
     return;
   }
-  seg_sample_block<T>(it.a.x, it.a.y, it.a.z, it.a.n, it.a.dim, it.seg_in, it.rel_mode, it.rel_eb, it.a.eb,
-                      (it.flags & kBatchSafe31) ? 1 : 0, it.a.ctl, blockIdx.x, gridDim.x);
+  seg_sample_block<T>(it.a.x, it.a.y, it.a.z, it.a.n, it.a.dim, it.seg_in, (it.flags & kBatchRelMode) ? 1 : 0, it.rel_eb, it.a.eb,
+                      (it.flags & kBatchSafe31) ? 1 : 0, it.a.ctl, blockIdx.x, gridDim.x, nullptr, &it.seg);
 }
 
-template <int W>
-struct BatchGroup {
-  uint32_t sz[W];             // payload bytes of each warp's chunk
-  unsigned long long goff;    // stream offset of the group (~0: look-back gave up)
-  unsigned long long next;    // next global group
-  unsigned long long nmap;    // its map entry
+// A CTA's view of the work list: the chunk of the current and of the next
+// iteration (by parity), with their snapshots' arguments, and the parked
+// payloads' arguments by slot.
+template <typename T>
+struct BatchState {
+  CArgs<T> args[2];
+  CArgs<T> parked[kEncSlots];
+  unsigned long long chunk[2];  // chunk within the snapshot (>= G: past the list's end)
+  uint32_t seg[2];
 };
 
-// The compress loop of compress_kernel over a work list of many snapshots:
-// map[g] = snapshot << 40 | group of global group g.  The arguments of the
-// current and the next group's snapshot live in shared memory (double
-// buffered: the next group's points are loaded before the current group's
-// copy-out).  A snapshot whose segment size could not be chosen (sampling
-// error, status set) is skipped as a whole.  Groups of W chunks, as in
-// compress_kernel<T, DIM>.
-template <typename T, int DIM, int W = enc_warps<T, DIM>()>
-__global__ void __launch_bounds__(32 * W, GPZ_ENC_MIN_CTAS)
-    compress_batch_kernel(const BItem<T> *__restrict__ items, const unsigned long long *__restrict__ map,
-                          unsigned long long total, unsigned long long *claim) {
-  using Tr = TT<T>;
+// One warp copies a snapshot's arguments.
+template <typename T>
+__device__ __forceinline__ void copy_args(CArgs<T> &dst, const CArgs<T> &src, int lane) {
+  constexpr int W = (int)(sizeof(CArgs<T>) / 4);
+  static_assert(sizeof(CArgs<T>) % 4 == 0 && W <= 32, "one word per lane");
+  if (lane < W) reinterpret_cast<uint32_t *>(&dst)[lane] = reinterpret_cast<const uint32_t *>(&src)[lane];
+}
+
+// The last of the K snapshots whose first chunk is at or below g (a warp
+// probes 32 of them per step).
+template <typename T>
+__device__ __forceinline__ uint32_t find_item(const BItem<T> *items, uint32_t K, unsigned long long g, int lane) {
+  uint32_t lo = 0, len = K;
+  while (len > 1) {
+    const uint32_t step = (len + 31) / 32, i = lo + lane * step;
+    const bool in = lane * step < len && items[i].start <= g;
+    const int top = 31 - __clz((int)__ballot_sync(0xFFFFFFFFu, in));  // lane 0 always holds
+    len = min(step, len - top * step);
+    lo += top * step;
+  }
+  return lo;
+}
+
+// The compress loop of compress_kernel over the chunks of many snapshots.  A
+// snapshot whose segment size could not be chosen (sampling error, status
+// set) is skipped as a whole.
+template <typename T, int DIM>
+__global__ void __launch_bounds__(kEncThreads, kEncCtas)
+    compress_batch_kernel(const BItem<T> *items, uint32_t K, unsigned long long total, unsigned long long *claim) {
   constexpr bool is64 = sizeof(T) == 8;
-  constexpr uint32_t FULL = 0xFFFFFFFFu;
-  constexpr unsigned long long kLocal = (1ull << kBatchLocalBits) - 1;
-  extern __shared__ __align__(16) uint32_t enc_smem[];
-  __shared__ BatchGroup<W> eg;
-  __shared__ CArgs<T> args[2];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t *const sw = enc_smem + warp * kEncWords;
-  auto claim_next = [&](int slot) {  // thread 0
-    const unsigned long long g = atomicAdd(claim, 1ull);
-    eg.next = g;
-    // past the end: the first snapshot's first group stands in, so the
-    // prefetch below needs no condition (its loads are never used)
-    const unsigned long long m = g < total ? map[g] : 0ull;
-    eg.nmap = m;
-    args[slot] = items[m >> kBatchLocalBits].a;
+  extern __shared__ __align__(16) unsigned char enc_smem[];
+  EncShared &sm = *reinterpret_cast<EncShared *>(enc_smem);
+  __shared__ BatchState<T> bs;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  unsigned long long claimed = 0;
+  auto claim_next = [&]() {  // one warp
+    if (lane == 0) claimed = atomicAdd(claim, 1ull);
   };
-  if (threadIdx.x == 0) claim_next(0);
+  auto fetch = [&](int slot) {  // the same warp, later
+    const unsigned long long g = __shfl_sync(0xFFFFFFFFu, claimed, 0);
+    if (lane == 0) sm.next[slot] = g;
+    if (g >= total) return;
+    const BItem<T> &it = items[find_item(items, K, g, lane)];
+    copy_args(bs.args[slot], it.a, lane);
+    if (lane == 0) {
+      bs.chunk[slot] = g - it.start;
+      bs.seg[slot] = it.seg;
+    }
+    prefetch_points<T, DIM>(it.a, g - it.start, lane);
+  };
+  if (t == 0) sm.overflowed = nullptr;
+  if (warp == 2) {
+    claim_next();
+    fetch(0);
+  }
   __syncthreads();
-  ChunkPoints<T, DIM> pts;
-  pts.load(args[0], (eg.nmap & kLocal) * W + warp, lane);
-  int slot = 0;
-  uint32_t rank_skip = 0;
+  Parked pk = {0u, 0u};
+  uint32_t rank_skip = 0, declined = 0;
+  int par = 0;
   for (;;) {
-    const unsigned long long g = eg.next;
-    if (g >= total) break;
-    const unsigned long long m = eg.nmap;
-    __syncthreads();  // B0: everyone has the group before it is replaced
-    if (threadIdx.x == 0) claim_next(slot ^ 1);
-    const CArgs<T> &a = args[slot];
-    Control *ctl = a.ctl;
-    const unsigned long long G = a.G;
-    const unsigned long long gid = m & kLocal, gbase = gid * W;
-    const uint32_t seg = ctl->seg;  // 0: the snapshot's sampling failed
-    const bool live = seg != 0;
-    const uint32_t sh = live ? (uint32_t)__ffs((int)seg) - 1u : 0u, msk = seg - 1u;
+    if (sm.next[par] >= total) break;
+    const unsigned long long c = bs.chunk[par];
+    const uint32_t seg = bs.seg[par];
+    if (seg == 0u) {  // the snapshot's sampling failed
+      __syncthreads();
+      if (warp == 2) {
+        claim_next();
+        fetch(par ^ 1);
+      }
+      __syncthreads();
+      par ^= 1;
+      continue;
+    }
+    const CArgs<T> &a = bs.args[par];
     const T eb = a.eb;
     const T inv = is64 ? (T)__ddiv_rn(1.0, __dmul_rn(2.0, (double)eb)) : (T)__fdiv_rn(1.0f, __fmul_rn(2.0f, (float)eb));
-    const unsigned long long pay_base = Tr::hdr + 8ull * G + (unsigned long long)Tr::meta * G;
-    const unsigned long long c = gbase + warp;
-    uint32_t tot = 0;
-    auto on_size = [&](uint32_t bytes) {
-      if (lane == 0) eg.sz[warp] = bytes;
-      __syncthreads();  // B1: the group's sizes are known (and the next group's snapshot)
-      if (live && warp == 0) {
-        const uint32_t s = lane < W ? eg.sz[lane] : 0u;
-        tot = __reduce_add_sync(FULL, s);
-        if (lane == 0) publish_aggregate(a.look, gid, tot);
-      }
-    };
-    uint32_t payload = 0, meta_word = 0;
-    if (live && c < G) payload = encode_chunk<T, DIM>(a, c, sw, seg, sh, msk, eb, inv, pts, meta_word, lane, rank_skip, on_size);
-    else on_size(0u);
-    if (live && warp == 0) {
-      unsigned long long excl = 0;
-      const bool ok = resolve_prefix(a.look, gid, tot, ctl, excl);
-      if (lane == 0) eg.goff = ok ? excl : ~0ull;
+    const uint32_t slot = encode_chunk<T, DIM>(a, c, sm, par, seg, eb, inv, bs.parked, pk, rank_skip, declined, claim_next,
+                                               [&]() { fetch(par ^ 1); });
+    // the next look-up is the first warp's, before a barrier
+    if (warp == 0) {
+      copy_args(bs.parked[slot], a, lane);
+      __syncwarp();
     }
-    pts.load(args[slot ^ 1], (eg.nmap & kLocal) * W + warp, lane);  // in flight during the copy-out
-    __syncthreads();  // B2: the group's stream offset is known
-    const unsigned long long goff = eg.goff;
-    if (live && c < G && goff != ~0ull) {
-      unsigned long long off = goff;
-      for (int w = 0; w < warp; ++w) off += eg.sz[w];
-      place_chunk<T>(a, c, G, pay_base, off, payload, meta_word, seg, eb, sw, lane);
-    }
-    slot ^= 1;
+    par ^= 1;
   }
+  flush_parked<T>(bs.parked, sm, pk, lane, warp);
 }
 
 // ---------------------------------------------------------------------------

@@ -32,15 +32,9 @@ inline uint64_t align256(uint64_t v) { return (v + 255u) & ~255ull; }
 inline uint64_t chunks_of(uint64_t n) { return (n + kChunk - 1) / kChunk; }
 inline uint64_t rel_blocks_of(uint64_t n) { return std::min(kRelMaxBlocks, std::max<uint64_t>(1, n / kRelPointsPerBlock)); }
 int class_of(uint32_t bits, uint32_t dim) { return (bits == 64 ? 2 : 0) + (dim == 3 ? 1 : 0); }
-// chunks per group of a class's compress kernel (enc_warps of its float type and dimension)
-constexpr int class_warps(int c) {
-  return c == 0 ? enc_warps<float, 2>() : c == 1 ? enc_warps<float, 3>() : c == 2 ? enc_warps<double, 2>() : enc_warps<double, 3>();
-}
-inline uint64_t groups_of(uint64_t n, int c) { return (chunks_of(n) + class_warps(c) - 1) / class_warps(c); }
-
 template <typename T>
-void fill_item(BItem<T> &bi, const gpz_batch_item &it, uint8_t *dev, uint64_t ctl_off, uint64_t rctl_off,
-               uint64_t look_off) {
+void fill_item(BItem<T> &bi, const gpz_batch_item &it, uint8_t *dev, uint64_t ctl_off, uint64_t look_off,
+               uint64_t start) {
   memset(&bi, 0, sizeof(bi));
   bi.a.x = static_cast<const T *>(it.d_x);
   bi.a.y = static_cast<const T *>(it.d_y);
@@ -48,20 +42,17 @@ void fill_item(BItem<T> &bi, const gpz_batch_item &it, uint8_t *dev, uint64_t ct
   bi.a.out = static_cast<uint8_t *>(it.d_out);
   bi.a.out_cap = it.out_capacity;
   bi.a.ctl = reinterpret_cast<Control *>(dev + ctl_off);
-  bi.a.look = reinterpret_cast<unsigned long long *>(dev + look_off);
+  bi.a.look = reinterpret_cast<unsigned long long *>(dev + look_off - 32)  /* record 1 lies at look + 32 */;
   bi.a.n = it.n;
   bi.a.G = chunks_of(it.n);
   bi.a.eb = (T)it.eb;
   bi.a.eb_dev = nullptr;
   bi.a.dim = it.dim;
-  auto al = [](const void *p) { return ((uintptr_t)p & 15u) == 0; };
-  bi.a.vec_ok = al(it.d_x) && al(it.d_y) && (it.dim == 2 || al(it.d_z));
-  bi.rctl = reinterpret_cast<Control *>(dev + rctl_off);
+  bi.start = start;
   bi.rel_eb = (T)it.rel_eb;
   bi.seg_in = it.seg_size;
-  bi.rel_mode = it.rel_mode;
   bi.flags = ((it.flags & GPZ_FLAG_SEG_FIXED) ? kBatchSegFixed : 0u) | ((it.flags & GPZ_FLAG_SAFE31) ? kBatchSafe31 : 0u) |
-             ((it.flags & GPZ_FLAG_REL_ON_DEVICE) ? kBatchRelDev : 0u);
+             ((it.flags & GPZ_FLAG_REL_ON_DEVICE) ? kBatchRelDev : 0u) | (it.rel_mode ? kBatchRelMode : 0u);
 }
 
 template <typename T>
@@ -85,20 +76,22 @@ void fill_ditem(DItem<T> &d, const gpz_dbatch_item &it, Control *ctl) {
 // exactly gpz_rel_to_abs's (min and max do not depend on the partition) and
 // goes to the snapshot's descriptor, where sampling and compress read it.
 template <typename T>
-__global__ void __launch_bounds__(256) batch_rel_mapped_kernel(BItem<T> *items, const unsigned long long *rmap) {
+__global__ void __launch_bounds__(256, 6) batch_rel_mapped_kernel(BItem<T> *items, const unsigned long long *rmap,
+                                                                 uint32_t count) {
   const unsigned long long e = rmap[blockIdx.x];
   BItem<T> &it = items[e >> 40];
+  // the snapshot's second control block, `count` blocks behind its first
+  Control *rctl = reinterpret_cast<Control *>(reinterpret_cast<uint8_t *>(it.a.ctl) + (size_t)count * kCtlBytes);
   const unsigned nb = (unsigned)((e >> 20) & 0xFFFFFu), b = (unsigned)(e & 0xFFFFFu);
-  rel_to_abs_block<T>(it.a.x, it.a.y, it.a.z, it.a.n, it.a.dim, it.rel_eb, it.rctl, &it.a.eb, b, nb);
+  rel_to_abs_block<T>(it.a.x, it.a.y, it.a.z, it.a.n, it.a.dim, it.rel_eb, rctl, &it.a.eb, b, nb);
 }
 
 // Grids of the batched persistent kernels on the current device (-1 when the
 // kernel's shared-memory attribute cannot be raised there).
 template <typename T, int DIM>
-int compress_grid(uint64_t groups) {
-  constexpr int W = enc_warps<T, DIM>();
-  const int o = resident_ctas(compress_batch_kernel<T, DIM>, 32 * W, enc_smem_bytes<W>());
-  return o ? (int)std::min<uint64_t>(groups, (uint64_t)current_sms() * o) : -1;
+int compress_grid(uint64_t chunks) {
+  const int o = resident_ctas(compress_batch_kernel<T, DIM>, kEncThreads, sizeof(EncShared));
+  return o ? (int)std::min<uint64_t>(chunks, (uint64_t)current_sms() * o) : -1;
 }
 
 template <typename T, int DIM, class Cfg = DecCfg<T>, int PASS = kPassAll>
@@ -109,16 +102,14 @@ int dec_grid(uint64_t chunks) {
 }
 
 template <typename T, int DIM>
-void enqueue_class(const gpzb_host::ClassPlan &cp, uint8_t *dev, uint64_t claim_off, cudaStream_t st) {
+void enqueue_class(const gpzb_host::ClassPlan &cp, uint32_t count, uint8_t *dev, uint64_t claim_off, cudaStream_t st) {
   BItem<T> *tab = reinterpret_cast<BItem<T> *>(dev + cp.table_off);
   if (cp.rel_blocks)
     batch_rel_mapped_kernel<T><<<(unsigned)cp.rel_blocks, 256, 0, st>>>(
-        tab, reinterpret_cast<const unsigned long long *>(dev + cp.rmap_off));
+        tab, reinterpret_cast<const unsigned long long *>(dev + cp.rmap_off), count);
   batch_sample_kernel<T><<<dim3(128, (unsigned)cp.items.size()), 256, 0, st>>>(tab);
-  constexpr int W = enc_warps<T, DIM>();
-  compress_batch_kernel<T, DIM><<<cp.grid, 32 * W, enc_smem_bytes<W>(), st>>>(
-      tab, reinterpret_cast<const unsigned long long *>(dev + cp.map_off), cp.work,
-      reinterpret_cast<unsigned long long *>(dev + claim_off));
+  compress_batch_kernel<T, DIM><<<cp.grid, kEncThreads, sizeof(EncShared), st>>>(
+      tab, (uint32_t)cp.items.size(), cp.work, reinterpret_cast<unsigned long long *>(dev + claim_off));
 }
 
 template <typename T, int DIM>
@@ -165,10 +156,10 @@ bool compress_layout(const gpz_batch_item *items, uint32_t count, Layout &L) {
   for (uint32_t i = 0; i < count; ++i) {
     L.look_off[i] = off;
     const int c = class_of(items[i].float_bits, items[i].dim);
-    off += 8 * groups_of(items[i].n, c);
+    off += look_bytes(chunks_of(items[i].n));
     ClassPlan &cp = L.cls[c];
     cp.items.push_back(i);
-    cp.work += groups_of(items[i].n, c);
+    cp.work += chunks_of(items[i].n);
     if (items[i].flags & GPZ_FLAG_REL_ON_DEVICE) cp.rel_blocks += rel_blocks_of(items[i].n);
   }
   L.claim_off = align256(off);
@@ -179,8 +170,6 @@ bool compress_layout(const gpz_batch_item *items, uint32_t count, Layout &L) {
     if (cp.items.empty()) continue;
     cp.table_off = off;
     off = align256(off + (c < 2 ? sizeof(BItem<float>) : sizeof(BItem<double>)) * cp.items.size());
-    cp.map_off = off;
-    off = align256(off + 8 * cp.work);
     cp.rmap_off = off;
     off = align256(off + 8 * cp.rel_blocks);
     switch (c) {
@@ -235,18 +224,16 @@ void compress_tables(const gpz_batch_item *items, const Layout &L, uint8_t *dev,
   for (int c = 0; c < 4; ++c) {
     const ClassPlan &cp = L.cls[c];
     if (cp.items.empty()) continue;
-    uint64_t g = 0, rb = 0;
-    unsigned long long *map = reinterpret_cast<unsigned long long *>(H(cp.map_off));
+    uint64_t start = 0, rb = 0;
     unsigned long long *rmap = reinterpret_cast<unsigned long long *>(H(cp.rmap_off));
     for (size_t k = 0; k < cp.items.size(); ++k) {
       const uint32_t i = cp.items[k];
       const gpz_batch_item &it = items[i];
       if (c < 2) fill_item<float>(reinterpret_cast<BItem<float> *>(H(cp.table_off))[k], it, dev, ctl_off(i),
-                                  ctl_off(L.count + i), L.look_off[i]);
+                                  L.look_off[i], start);
       else fill_item<double>(reinterpret_cast<BItem<double> *>(H(cp.table_off))[k], it, dev, ctl_off(i),
-                             ctl_off(L.count + i), L.look_off[i]);
-      const uint64_t groups = groups_of(it.n, c);
-      for (uint64_t q = 0; q < groups; ++q) map[g++] = ((unsigned long long)k << kBatchLocalBits) | q;
+                             L.look_off[i], start);
+      start += chunks_of(it.n);
       if (it.flags & GPZ_FLAG_REL_ON_DEVICE) {
         const uint64_t nb = rel_blocks_of(it.n);
         for (uint64_t q = 0; q < nb; ++q) rmap[rb++] = ((unsigned long long)k << 40) | (nb << 20) | q;
@@ -279,10 +266,10 @@ void compress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st) {
     if (L.cls[c].items.empty()) continue;
     const uint64_t claim = L.claim_off + 8ull * c;
     switch (c) {
-      case 0: enqueue_class<float, 2>(L.cls[c], dev, claim, st); break;
-      case 1: enqueue_class<float, 3>(L.cls[c], dev, claim, st); break;
-      case 2: enqueue_class<double, 2>(L.cls[c], dev, claim, st); break;
-      default: enqueue_class<double, 3>(L.cls[c], dev, claim, st); break;
+      case 0: enqueue_class<float, 2>(L.cls[c], L.count, dev, claim, st); break;
+      case 1: enqueue_class<float, 3>(L.cls[c], L.count, dev, claim, st); break;
+      case 2: enqueue_class<double, 2>(L.cls[c], L.count, dev, claim, st); break;
+      default: enqueue_class<double, 3>(L.cls[c], L.count, dev, claim, st); break;
     }
   }
 }

@@ -60,8 +60,9 @@ int compress_t(const gpz_params *p, const void *d_x, const void *d_y, const void
   if (out_capacity < Tr::hdr + G * (8ull + Tr::meta)) return GPZ_ENOSPACE;
   if (scratch_bytes < gpz_compress_scratch_bytes(p->n)) return GPZ_ENOSPACE;
   Control *ctl = static_cast<Control *>(d_scratch);
-  unsigned long long *look = reinterpret_cast<unsigned long long *>(static_cast<uint8_t *>(d_scratch) + kCtlBytes);
-  cudaError_t e = cudaMemsetAsync(d_scratch, 0, kCtlBytes + 8ull * G, st);
+  // the look-back records: the first in the control block, the others behind it
+  unsigned long long *look = reinterpret_cast<unsigned long long *>(static_cast<uint8_t *>(d_scratch) + kLookTail);
+  cudaError_t e = cudaMemsetAsync(d_scratch, 0, kCtlBytes + look_bytes(G), st);
   if (e != cudaSuccess) return GPZ_ECUDA;
   const T eb = (T)p->eb;
   const T rel = (T)p->rel_eb;
@@ -91,21 +92,16 @@ int compress_t(const gpz_params *p, const void *d_x, const void *d_y, const void
   a.eb = eb;
   a.eb_dev = eb_dev;
   a.dim = p->dim;
-  a.vec_ok = aligned16(d_x) && aligned16(d_y) && (p->dim == 2 || aligned16(d_z));
-  // persistent grid: one CTA per W chunks in flight (W = enc_warps<T, DIM>)
+  // persistent grid: one CTA per chunk in flight
   NvtxRange krange("run compress kernel");
-  auto launch = [&](auto kernel, auto w) -> bool {
-    constexpr int W = decltype(w)::value;
-    constexpr size_t smem = enc_smem_bytes<W>();
-    const int occ = resident_ctas(kernel, 32 * W, smem);
+  auto launch = [&](auto kernel) -> bool {
+    const int occ = resident_ctas(kernel, kEncThreads, sizeof(EncShared));
     if (occ == 0) return false;
-    const uint64_t grid = std::min<uint64_t>((G + W - 1) / W, (uint64_t)num_sms() * occ);
-    kernel<<<(unsigned)grid, 32 * W, smem, st>>>(a);
+    const uint64_t grid = std::min<uint64_t>(G, (uint64_t)num_sms() * occ);
+    kernel<<<(unsigned)grid, kEncThreads, sizeof(EncShared), st>>>(a);
     return true;
   };
-  using W3 = std::integral_constant<int, enc_warps<T, 3>()>;
-  using W2 = std::integral_constant<int, enc_warps<T, 2>()>;
-  if (!(p->dim == 3 ? launch(compress_kernel<T, 3>, W3{}) : launch(compress_kernel<T, 2>, W2{}))) return GPZ_ECUDA;
+  if (!(p->dim == 3 ? launch(compress_kernel<T, 3>) : launch(compress_kernel<T, 2>))) return GPZ_ECUDA;
   return cuda_status(cudaGetLastError());
 }
 
@@ -558,10 +554,10 @@ int gpz_compress_noalloc(const gpz_params *params, const void *d_x, const void *
 // the CTA holding it had stopped), so the wait runs out after `polls` polls.
 // ---------------------------------------------------------------------------
 namespace {
-__global__ void lookback_timeout_kernel(unsigned long long *look, Control *ctl, uint32_t polls) {
+__global__ void lookback_timeout_kernel(Control *ctl, uint32_t polls) {
   unsigned long long excl = 0;
-  const bool ok = resolve_prefix(look, 1ull, 0ull, ctl, excl, polls);
-  if (threadIdx.x == 0) ctl->stream_bytes = ok ? 1ull : 0ull;
+  const int ok = resolve_prefix(ctl, nullptr, 1ull, excl, polls);  // record 0 only
+  if (threadIdx.x == 0) ctl->stream_bytes = ok > 0 ? 1ull : 0ull;
 }
 }  // namespace
 
@@ -571,9 +567,8 @@ extern "C" int gpz_selftest_lookback_timeout(uint32_t polls, void *d_scratch, ui
   if (scratch_bytes < kCtlBytes + 16) return GPZ_ENOSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Control *ctl = static_cast<Control *>(d_scratch);
-  unsigned long long *look = reinterpret_cast<unsigned long long *>(static_cast<uint8_t *>(d_scratch) + kCtlBytes);
   if (cudaMemsetAsync(d_scratch, 0, kCtlBytes + 16, st) != cudaSuccess) return GPZ_ECUDA;
-  lookback_timeout_kernel<<<1, 32, 0, st>>>(look, ctl, polls);
+  lookback_timeout_kernel<<<1, 32, 0, st>>>(ctl, polls);
   if (cudaGetLastError() != cudaSuccess) return GPZ_ECUDA;
   Control h;
   if (cudaMemcpyAsync(&h, d_scratch, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess) return GPZ_ECUDA;

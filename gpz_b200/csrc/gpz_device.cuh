@@ -8,6 +8,7 @@
 // that places each group's payloads directly in the output stream.
 #pragma once
 
+#include <cfloat>
 #include <cstdint>
 #include <cstring>
 #include <cuda_runtime.h>
@@ -128,6 +129,46 @@ __device__ __forceinline__ float fmax3f(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
+}
+
+// Warp-wide float min / max in one instruction each (sm_100a's redux.f32):
+// NaN sources ignored, -0.0 below +0.0, as the two-input forms.
+__device__ __forceinline__ float warp_fmin(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_fmax(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// Minimum and maximum of a warp's N values per lane, from the type's limits
+// on (a warp of NaNs keeps them).
+template <int N>
+__device__ __forceinline__ void warp_minmax(const float (&v)[N], float &mn, float &mx) {
+  mn = FLT_MAX;
+  mx = -FLT_MAX;
+#pragma unroll
+  for (int e = 0; e < N; e += 2) {
+    mn = fmin3f(mn, v[e], v[e + 1]);
+    mx = fmax3f(mx, v[e], v[e + 1]);
+  }
+  mn = warp_fmin(mn);
+  mx = warp_fmax(mx);
+}
+template <int N>
+__device__ __forceinline__ void warp_minmax(const double (&v)[N], double &mn, double &mx) {
+  mn = DBL_MAX;
+  mx = -DBL_MAX;
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    mn = fmin(mn, v[e]);
+    mx = fmax(mx, v[e]);
+  }
+  mn = from_ord(~warp_max(~ord_of(mn)));
+  mx = from_ord(warp_max(ord_of(mx)));
 }
 
 __device__ __forceinline__ uint32_t bitlen(uint32_t v) { return 32u - (uint32_t)__clz(v); }
@@ -380,13 +421,16 @@ struct FastDiv31 {
   }
 };
 
-// Relaxed GPU-scope accesses for the look-back words.
-__device__ __forceinline__ void st_relaxed(unsigned long long *p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+// Relaxed GPU-scope accesses for the look-back records.
+__device__ __forceinline__ void red_or_relaxed(unsigned long long *p, unsigned long long v) {
+  asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long *p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+__device__ __forceinline__ uint4 ld_relaxed4(const uint4 *p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
   return v;
 }
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p) { return *(const volatile uint32_t *)p; }

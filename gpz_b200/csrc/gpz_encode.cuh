@@ -5,30 +5,36 @@
 //                     1620-1702; float64 twin src/cudaWarpCompressDouble.cu)
 //                     fused into one persistent, single-pass kernel.
 //
-// One warp encodes one 1024-point chunk.  Lane l holds the 32 points whose
-// stable rank r(p) = (p % 32) * 32 + p / 32 (the reference's sort order for
-// equal block ids) is 32l..32l+31, so the composite (block id, r) is unique
-// and a point's register index is its rank within the lane.  The warp:
-//   1. loads and quantizes one axis at a time (block id in registers, the
-//      relative position accumulated in a shared row per lane);
-//   2. ranks the composites (block id - kmin) << 10 | r through 2048 buckets
-//      on their top bits (shared-atomic counts, placement by bucket start +
-//      arrival slot, multi-point buckets put in order afterwards) when they
-//      span 21 bits or more; a data-independent warp sort of the 1024 values
-//      (odd-even merge sort of each lane's 32, then bitonic merges across
-//      lanes on the transposed matrix) ranks narrower ones and the 32-bit
-//      chunks the buckets decline;
-//   3. finds the runs of equal ids (unique ids, deltas, counts) and compacts
-//      them through shared memory so lane l holds runs 32l..32l+31;
-//   4. reports its payload size, then transposes deltas, counts and relative
-//      positions into bit planes in registers and assembles the payload in
-//      its shared region.
-// The 8 warps of a CTA take 8 consecutive chunks (a group) together, with
-// three CTA barriers per group: B0 before the next group is claimed, B1 once
-// every payload size is known (warp 0 then publishes the group's aggregate),
-// B2 once warp 0, after building its own planes, has resolved the group's
-// stream offset (one decoupled look-back per group); each warp then copies
-// its payload out while the next chunk's loads are in flight.
+// A CTA of four warps encodes one 1024-point chunk at a time, eight points a
+// thread.  The stable rank of point p among equal block ids is
+// r(p) = (p % 32) * 32 + p / 32, so the composite (block id, r) is unique and
+// any correct sort reproduces the reference's order.  Per chunk:
+//   1. load the points, the chunk's min / max; quantize (block id in registers,
+//      relative position in shared memory); place the oldest parked payload,
+//      whose stream offset the last warp looks up while the first one works
+//      out the chunk's scalars;
+//   2. rank: 1024 buckets over the id range (shared-atomic counts, scan,
+//      placement at bucket start + arrival slot, then odd-even transposition
+//      between neighbouring positions); a chunk with few distinct ids or a
+//      crowded bucket goes through a stable radix sort instead;
+//   3. runs of equal ids (unique ids, deltas, counts), the payload's size,
+//      which is published at once for the chunks behind;
+//   4. bit planes, eight at a time per warp, into a staged payload, which
+//      stays parked in shared memory until a later chunk's step 1 or 3.
+//
+// What bounds it: instruction issue (55 %) and shared-memory wavefronts (58 %)
+// with the barriers between the steps on top; HBM needs a quarter of the time.
+// One warp a chunk with 32 points a lane (128-168 registers, 12-16 warps an
+// SM, payloads placed behind CTA barriers) issued 42 % and took a chunk's whole
+// latency, some 50 us, on any input: this form takes 18 against 63 us on 5,003
+// float 3D points, 0.75 against 1.06 ms on 50M double 3D points of a lattice,
+// 1.48 against 1.55 ms on the 143.7M-point clustered snapshot, 0.36 against
+// 0.42 ms on 32M uniform points.
+//
+// Two parked payloads a CTA: a payload can be placed once all chunks before it
+// have published their sizes, and CTAs differ by tens of percent from chunk to
+// chunk.  With room for one (8 CTAs an SM) nine in ten look-ups had to wait,
+// with two (6 CTAs) one in twenty.
 #pragma once
 
 #include <cfloat>
@@ -37,68 +43,24 @@
 
 namespace gpzb {
 
-#ifndef GPZ_ENC_MIN_CTAS
-#define GPZ_ENC_MIN_CTAS 2                // resident CTAs per SM the register budget is sized for
-#endif
-#ifndef GPZ_ENC_WARPS
-#define GPZ_ENC_WARPS 8
-#endif
-#ifndef GPZ_ENC_WARPS_F64_3D
-#define GPZ_ENC_WARPS_F64_3D 6
-#endif
-constexpr int kEncWarps = GPZ_ENC_WARPS;  // chunks (warps) per CTA
-constexpr int kEncBucketBits = 11;        // ranking buckets per chunk: 2048
-constexpr int kEncSmall = 16;             // buckets of this many points or more are sorted by the whole warp
-constexpr uint32_t kEncBucketBackoff = 8; // chunks ranked by the warp sort alone after a declined one
-constexpr int kEncWords = 3 * kChunk;     // per-warp shared words (12 KB)
-static_assert(kStageBytes <= kEncWords * 4, "payload staging must fit the warp region");
+constexpr int kEncThreads = 128;          // threads (one chunk) per CTA
+constexpr int kEncWarps = kEncThreads / 32;
+constexpr int kEncPer = kChunk / kEncThreads;  // points per thread
+constexpr int kEncBuckets = 1024;         // ranking buckets per chunk
+constexpr int kEncBucketBits = 11;        // id ranges below 2^11 skip the buckets
+constexpr int kEncSmall = 16;             // a bucket of this many points or more is sorted on its own
+constexpr int kEncCrowd = 256;            // one above this size declines the chunk, and so do more than
+constexpr int kEncCrowdPoints = 512;      //   this many points in all buckets of kEncSmall or more
+constexpr uint32_t kEncBucketBackoff = 8; // chunks sorted directly after two declined ones in a row
+constexpr int kEncSlots = 2;              // payloads a CTA can park
+constexpr int kEncCtas = 6;               // resident CTAs per SM (36 KB of shared memory each)
+constexpr int kEncHalo = 16;              // positions a warp orders beyond its own on either side
+constexpr int kEncOrd = 9;                // positions per lane while ordering: 32 * 9 = 256 + 2 * 16
+static_assert(kEncSlots >= 2, "the oldest payload is looked up while the newest is written");
+static_assert(kChunk / kEncWarps + 2 * kEncHalo == 32 * kEncOrd, "ordering window");
+static_assert(kEncHalo >= kEncSmall - 1, "a small bucket must fit the halo");
 
-// Chunks (warps) per CTA of compress_kernel<T, DIM>: float64 3D streams use
-// 6 (about 170 registers a thread, where 8 warps spill: FCC 200M 4.6 -> 4.1
-// ms), the others 8 (6 measured slower for float32 and float64 2D).
-template <typename T, int DIM>
-constexpr int enc_warps() { return (sizeof(T) == 8 && DIM == 3) ? GPZ_ENC_WARPS_F64_3D : kEncWarps; }
-
-// Per-CTA state of the group of W consecutive chunks a CTA encodes.
-template <int W>
-struct EncGroupT {
-  uint32_t sz[W];            // payload bytes of each warp's chunk
-  unsigned long long goff;   // stream offset of the group (~0: look-back gave up)
-  unsigned long long next;   // first chunk of the next group
-};
-
-template <int W = kEncWarps>
-constexpr size_t enc_smem_bytes() { return (size_t)W * kEncWords * 4; }
-
-// Index of bucket-count word w, position / run u, ... in a swizzled 1024-word
-// array (rows of 32 words, 16-byte quads XORed by the row).
-__device__ __forceinline__ uint32_t sx(uint32_t i) { return (uint32_t)swz((int)i); }
-
-// Ascending in-place bitonic sort of the n = hi - lo values a[sx(lo..hi)) by
-// one warp (variant whose exchanges all put the minimum at the lower index,
-// virtually padded with +inf up to a power of two).
-static __device__ void warp_bitonic_u32(uint32_t *a, uint32_t lo, uint32_t n, int lane) {
-  uint32_t P = 2;
-  while (P < n) P <<= 1;
-  for (uint32_t k = 2; k <= P; k <<= 1) {
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      for (uint32_t q = lane; q < (P >> 1); q += 32) {
-        const uint32_t i = ((q & ~(j - 1)) << 1) | (q & (j - 1));
-        const uint32_t p = (j == (k >> 1)) ? (i ^ (k - 1)) : (i + j);
-        if (p < n) {
-          const uint32_t x = a[sx(lo + i)], y = a[sx(lo + p)];
-          if (y < x) {
-            a[sx(lo + i)] = y;
-            a[sx(lo + p)] = x;
-          }
-        }
-      }
-      __syncwarp();
-    }
-  }
-}
-
-// Batcher's odd-even merge sort network on 32 registers (191 exchanges).
+// Batcher's odd-even merge sort network on 32 values (191 exchanges).
 __host__ __device__ __forceinline__ void oem_sort32(uint32_t (&a)[32]) {
 #pragma unroll
   for (int p = 1; p < 32; p <<= 1)
@@ -115,927 +77,977 @@ __host__ __device__ __forceinline__ void oem_sort32(uint32_t (&a)[32]) {
           }
 }
 
-__device__ __forceinline__ void cas_up(uint32_t &x, uint32_t &y) {
-  const uint32_t lo = min(x, y);
-  y = max(x, y);
-  x = lo;
+// Swizzled index of element i in a 1024-word array (see swz): rows of 32
+// words whose 16-byte quads are XORed by the row, so the plane jobs' row
+// reads (lane l: row l) and eight consecutive words per thread are free of
+// bank conflicts.
+__device__ __forceinline__ uint32_t sx(uint32_t i) { return (uint32_t)swz((int)i); }
+
+__device__ __forceinline__ float min2(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ float max2(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double min2(double a, double b) { return from_ord(min(ord_of(a), ord_of(b))); }
+__device__ __forceinline__ double max2(double a, double b) { return from_ord(max(ord_of(a), ord_of(b))); }
+
+// Index of rank r in a 1024-word array that is written by points (32 ranks a
+// row apart) and read in any order: the row's five bits XORed into the bank.
+__device__ __forceinline__ uint32_t rx(uint32_t r) { return r ^ (r >> 5); }
+
+// A CTA's shared memory.
+struct EncShared {
+  uint32_t A[2][kChunk];         // bucket counts -> sorted composites -> deltas | placed composites -> run starts
+                                 // (roles alternate from chunk to chunk: clearing the counts needs no barrier)
+  uint32_t R[kChunk];            // relative positions by point -> run lengths
+  uint32_t Q[kChunk];            // ranks in sorted order (not of narrow chunks) -> relative positions in that order
+  uint32_t P[kEncSlots][kStageBytes / 4];  // staged payloads
+  struct { unsigned long long c; uint32_t payload; } park[kEncSlots];  // their chunks and sizes
+  unsigned long long goff;       // stream offset of the parked chunk (kGoffPending, kGoffNone: none)
+  unsigned long long next[2];    // chunk claimed for the next iteration, by parity
+  __align__(16) double mm[kEncWarps][8];   // warps' minima (0..2) and maxima (4..6), in the stream's type
+  __align__(16) double nm[4];    // chunk: -min / (2 eb) per axis, in the stream's type
+  __align__(16) uint32_t sc[4];  // chunk: id multipliers of y and z, largest id
+  __align__(16) uint32_t tot[kEncWarps];   // per-warp sums of the bucket / digit scans
+  __align__(16) uint32_t big[kEncWarps];   // per-warp largest bucket
+  __align__(16) uint32_t relor[kEncWarps]; // OR of the relative positions
+  __align__(16) uint32_t seg[8 * kEncWarps];  // run starts per 32 positions: [warp][j]
+  __align__(16) uint32_t dor[kEncWarps];   // OR of the deltas
+  __align__(16) uint32_t cmax[kEncWarps];  // longest run
+  __align__(16) uint32_t cpts[kEncWarps];  // points in buckets of kEncSmall or more
+  __align__(16) uint32_t small[kEncWarps]; // per-warp largest bucket below that
+  uint32_t crowd[kEncCrowdPoints / kEncSmall];  // those buckets: first position << 16 | points
+  uint32_t ncrowd;
+  uint32_t first;                // smallest block id
+  Control *overflowed;           // stream whose id_overflow this CTA has set last
+};
+constexpr unsigned long long kGoffNone = ~0ull, kGoffPending = ~0ull - 1;
+
+__device__ __forceinline__ uint4 ld4(const uint32_t *p) { return *reinterpret_cast<const uint4 *>(p); }
+
+// One 32-element plane word of a delta / count section: bytes 4*lane.. of the
+// plane, MSB-first bit order (src/cudaWarpCompress.cu:357-408), only the
+// `room` bytes the plane has there.  Reversing the word's bits reverses the
+// order of its bytes too.
+__device__ __forceinline__ void put_plane_bytes(uint8_t *d, int room, uint32_t word) {
+  const uint32_t w = brev32(word);
+  if (room > 0) d[0] = (uint8_t)(w >> 24);
+  if (room > 1) d[1] = (uint8_t)(w >> 16);
+  if (room > 2) d[2] = (uint8_t)(w >> 8);
+  if (room > 3) d[3] = (uint8_t)w;
 }
 
-// Row <-> column transposes of the warp's 32x32 value matrix through a
-// 1024-word swizzled scratch (row l = lane l's registers).  Column reads and
-// writes touch one row per instruction, so all 32 banks; c[t] is the lane's
-// column offset inside rows with (row & 7) == t.
-__device__ __forceinline__ void column_offsets(uint32_t (&c)[8], int lane) {
+// Bit planes b0..b0+N-1 (those below nb; N = 8 or 16, b0 a multiple of 8) of a
+// 1024-element array (swizzled rows) by one warp: lane l takes elements
+// 32l..32l+31, gathers the N bits of each and turns them into plane words.
+// Planes go MSB plane first to byte pos0 of the staged payload: byte planes of
+// bpp bytes (bpp != 0) or planes of 32 words.
+template <int N>
+__device__ __forceinline__ void plane_job(const uint32_t *arr, uint8_t *stage, uint32_t pos0, uint32_t nb, uint32_t b0,
+                                          uint32_t bpp, int lane) {
+  uint32_t w[N];
+  const uint32_t k = b0 >> 3;
+  if constexpr (N == 8) {
+    const uint32_t s0 = k | ((4u + k) << 4);  // byte k of both sources
 #pragma unroll
-  for (int t = 0; t < 8; ++t) c[t] = ((uint32_t)(((lane >> 2) ^ t) & 7) << 2) + (lane & 3);
-}
-__device__ __forceinline__ void rows_to_columns(uint32_t (&v)[32], uint32_t *tsm, const uint32_t (&c)[8], int lane) {
-#pragma unroll
-  for (int m = 0; m < 8; ++m)
-    *reinterpret_cast<uint4 *>(tsm + qoff(lane, m)) = make_uint4(v[4 * m], v[4 * m + 1], v[4 * m + 2], v[4 * m + 3]);
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < 32; ++j) v[j] = tsm[32 * j + c[j & 7]];
-}
-__device__ __forceinline__ void columns_to_rows(uint32_t (&v)[32], uint32_t *tsm, const uint32_t (&c)[8], int lane) {
-#pragma unroll
-  for (int j = 0; j < 32; ++j) tsm[32 * j + c[j & 7]] = v[j];
-  __syncwarp();
-#pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const uint4 t = *reinterpret_cast<const uint4 *>(tsm + qoff(lane, m));
-    v[4 * m] = t.x; v[4 * m + 1] = t.y; v[4 * m + 2] = t.z; v[4 * m + 3] = t.w;
-  }
-}
-
-
-// Ascending sort of the warp's 1024 values held in the swizzled rows `rows`
-// (lane l: elements 32l..32l+31), in place; tsm is a second 1024-word scratch.  Bitonic sort in the variant whose comparators
-// all keep the minimum at the lower index: each merge of size k first pairs
-// mirrored elements (i, i ^ (k-1)), then (i, i + d) for d = k/4 .. 1.  Lanes
-// first sort their rows (odd-even merge network).  For k >= 64 the stages of
-// distance >= 32 run on the transposed matrix (lane L holding elements
-// 32j + L), where distance-d pairs are registers j, j + d/32 and the mirrored
-// pairs are register j ^ (k/32 - 1) of lane 31 - L.
-static __device__ __noinline__ void warp_sort1024_rows(uint32_t *rows, uint32_t *tsm, int lane) {
-  constexpr uint32_t FULL = 0xFFFFFFFFu;
-  uint32_t v[32];
-#pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const uint4 t = *reinterpret_cast<const uint4 *>(rows + qoff(lane, m));
-    v[4 * m] = t.x; v[4 * m + 1] = t.y; v[4 * m + 2] = t.z; v[4 * m + 3] = t.w;
-  }
-  uint32_t c[8];
-  column_offsets(c, lane);
-  oem_sort32(v);
-#pragma unroll
-  for (int lk = 6; lk <= 10; ++lk) {
-    rows_to_columns(v, tsm, c, lane);
-    {
-      const int mk = (1 << (lk - 5)) - 1, hb = 1 << (lk - 6);
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if ((j & hb) == 0) {
-          const int jj = j ^ mk;
-          const uint32_t pj = __shfl_xor_sync(FULL, v[jj], 31), pjj = __shfl_xor_sync(FULL, v[j], 31);
-          v[j] = min(v[j], pj);
-          v[jj] = max(v[jj], pjj);
-        }
+    for (int h = 0; h < 2; ++h) {
+      // quads h, h+2, h+4, h+6 of the row: elements 4h.. (+0, +8, +16, +24)
+      const uint4 q0 = ld4(arr + qoff(lane, h)), q1 = ld4(arr + qoff(lane, h + 2));
+      const uint4 q2 = ld4(arr + qoff(lane, h + 4)), q3 = ld4(arr + qoff(lane, h + 6));
+      w[4 * h + 0] = prmt(prmt(q0.x, q1.x, s0), prmt(q2.x, q3.x, s0), 0x5410);
+      w[4 * h + 1] = prmt(prmt(q0.y, q1.y, s0), prmt(q2.y, q3.y, s0), 0x5410);
+      w[4 * h + 2] = prmt(prmt(q0.z, q1.z, s0), prmt(q2.z, q3.z, s0), 0x5410);
+      w[4 * h + 3] = prmt(prmt(q0.w, q1.w, s0), prmt(q2.w, q3.w, s0), 0x5410);
     }
-#pragma unroll
-    for (int s = lk - 2; s >= 5; --s) {
-      const int dj = 1 << (s - 5);
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if ((j & dj) == 0) cas_up(v[j], v[j | dj]);
-    }
-    columns_to_rows(v, tsm, c, lane);
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1)
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if ((j & d) == 0) cas_up(v[j], v[j | d]);
-  }
-#pragma unroll
-  for (int m = 0; m < 8; ++m)
-    *reinterpret_cast<uint4 *>(rows + qoff(lane, m)) = make_uint4(v[4 * m], v[4 * m + 1], v[4 * m + 2], v[4 * m + 3]);
-}
-
-// Start of bucket b (b = 2048 gives the number of ranked points).
-__device__ __forceinline__ uint32_t bucket_start(const uint32_t *hist, uint32_t b, uint32_t total) {
-  if (b >= (1u << kEncBucketBits)) return total;
-  return (hist[sx(b >> 1)] >> ((b & 1u) << 4)) & 0xFFFFu;
-}
-
-// Writes one 32-element plane word of a delta / count section into the
-// staged payload: bytes 4*lane.. of the plane, MSB-first bit order
-// (src/cudaWarpCompress.cu:357-408), only the bytes the plane has.
-__device__ __forceinline__ void put_plane_bytes(uint8_t *stage8, uint32_t pos, uint32_t bpp, uint32_t word,
-                                                int lane) {
-  const int room = (int)bpp - 4 * lane;
-  if (room <= 0) return;
-  const uint32_t w = to_msb_bytes(word);
-  uint8_t *d = stage8 + pos + 4u * lane;
-  d[0] = (uint8_t)w;
-  if (room > 1) d[1] = (uint8_t)(w >> 8);
-  if (room > 2) d[2] = (uint8_t)(w >> 16);
-  if (room > 3) d[3] = (uint8_t)(w >> 24);
-}
-
-// Bit planes of this lane's 32 values (v: value of element j) into the staged
-// payload: byte planes at pos0 + pi*bpp (bpp != 0) or 32-word planes at word
-// pos0/4 + 32*pi + lane (bpp == 0), MSB plane first.  v is clobbered.
-__device__ __forceinline__ void put_planes(uint32_t *stage, uint32_t pos0, uint32_t nb, uint32_t bpp,
-                                           uint32_t (&v)[32], int lane) {
-  uint8_t *stage8 = reinterpret_cast<uint8_t *>(stage);
-  auto put = [&](uint32_t b, uint32_t w) {
-    const uint32_t pi = nb - 1u - b;
-    if (bpp) put_plane_bytes(stage8, pos0 + pi * bpp, bpp, w, lane);
-    else stage[(pos0 >> 2) + 32u * pi + lane] = w;
-  };
-  if (nb <= 8) {
-    transpose_lo8(v);
-#pragma unroll
-    for (int b = 0; b < 8; ++b)
-      if ((uint32_t)b < nb) put(b, v[b]);
-  } else if (nb <= 16) {
-    transpose_lo16(v);
-#pragma unroll
-    for (int b = 0; b < 16; ++b)
-      if ((uint32_t)b < nb) put(b, v[b]);
   } else {
-    transpose32(v);
+    const uint32_t s0 = k ? 0x7632u : 0x5410u;  // half k/2 of both sources
 #pragma unroll
-    for (int b = 0; b < 32; ++b)
-      if ((uint32_t)b < nb) put(b, v[b]);
+    for (int h = 0; h < 4; ++h) {
+      // quads h, h+4: elements 4h.. and 16 + 4h..
+      const uint4 q0 = ld4(arr + qoff(lane, h)), q1 = ld4(arr + qoff(lane, h + 4));
+      w[4 * h + 0] = prmt(q0.x, q1.x, s0);
+      w[4 * h + 1] = prmt(q0.y, q1.y, s0);
+      w[4 * h + 2] = prmt(q0.z, q1.z, s0);
+      w[4 * h + 3] = prmt(q0.w, q1.w, s0);
+    }
+    byte_stage<16>(w);
+  }
+  low_stages<N>(w);
+  const uint32_t left = nb - b0;  // planes of this job (all N, or the top ones)
+  if (bpp) {
+    const int room = (int)bpp - 4 * lane;
+    uint8_t *d = stage + pos0 + (left - 1u) * bpp + 4u * lane;
+#pragma unroll
+    for (int b = 0; b < N; ++b) {
+      if ((uint32_t)b >= left) break;
+      put_plane_bytes(d, room, w[b]);
+      d -= bpp;
+    }
+  } else {
+    uint32_t *d = reinterpret_cast<uint32_t *>(stage + pos0) + 32u * (left - 1u) + lane;
+#pragma unroll
+    for (int b = 0; b < N; ++b) {
+      if ((uint32_t)b >= left) break;
+      d[-32 * b] = w[b];
+    }
   }
 }
 
-// Ranks the chunk's composites (block id - kmin) << 10 | r through buckets
-// on their top bits: shared-atomic counts (the old count is the point's
-// arrival slot), an exclusive scan to bucket starts, placement at bucket
-// start + slot, then the order inside the buckets by odd-even transposition
-// steps on the lanes' registers once the positions are loaded in order.
-// cbits is the composites' width.
-//  * kNarrow (21 <= cbits <= 32): 1024 buckets with a 32-bit counter each
-//    (the fewest instructions per point); S holds whole composites, so neighbours of
-//    different buckets are already in order and the steps compare values
-//    alone.  A chunk with a bucket of 16 or more points is declined (the
-//    data-independent warp sort ranks it instead): false is returned before
-//    the placement, with S unchanged.
-//  * wide (cbits > 32): 2048 buckets, two 16-bit counters a word (S keeps
-//    the bits below the bucket, and they must fit 32 bits); the bucket of
-//    every position is scattered beside it, and the steps compare within a
-//    bucket only; buckets of 16 or more points are sorted by the warp's
-//    bitonic network in S first.
-// On entry S's row l holds lane l's block ids; after a true return S's row l
-// holds the sorted block ids of positions 32l..32l+31 and the first 16 words
-// of hist's row l the ranks r of positions j, j+16 as 16-bit pairs.
-template <bool kNarrow>
-static __device__ __noinline__ bool rank_buckets(uint32_t *sw, uint32_t kmin, uint32_t cbits, uint32_t nvalid,
-                                                 int lane) {
-  constexpr uint32_t FULL = 0xFFFFFFFFu;
-  uint32_t *const S = sw, *const hist = sw + kChunk;
-  const bool full = nvalid == (uint32_t)kChunk;
-  uint32_t key[32], rp[16];
-#pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const uint4 t = *reinterpret_cast<const uint4 *>(S + qoff(lane, m));
-    key[4 * m] = t.x; key[4 * m + 1] = t.y; key[4 * m + 2] = t.z; key[4 * m + 3] = t.w;
-  }
-#pragma unroll
-  for (int m = 0; m < 8; ++m) *reinterpret_cast<uint4 *>(hist + qoff(lane, m)) = make_uint4(0u, 0u, 0u, 0u);
-  __syncwarp();
-  // narrow: 1024 buckets on the top 10 bits, one 32-bit counter each, S
-  // keeps the whole composite; wide: 2048 buckets on the top 11 bits, two
-  // 16-bit counters a word, S keeps the bits below the bucket
-  const uint32_t shb = cbits - kEncBucketBits, lowb = shb - 10u;
-  uint32_t bs[32];  // narrow: counter word << 10 | arrival slot; wide: bucket << 10 | arrival
-                    // slot, then position << 11 | bucket
-#pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    const uint32_t koff = key[j] - kmin;
-    bs[j] = 0;
-    if constexpr (kNarrow) {
-      key[j] = (koff << 10) | (32u * lane + j);
-      if (full || 32u * j + lane < nvalid) {
-        const uint32_t w = sx(key[j] >> (shb + 1u));
-        bs[j] = (w << 10) | atomicAdd(&hist[w], 1u);
-      }
-    } else {
-      const uint32_t b = koff >> lowb;
-      key[j] = ((koff & ((1u << lowb) - 1u)) << 10) | (32u * lane + j);
-      if (full || 32u * j + lane < nvalid) {
-        const uint32_t h = (b & 1u) << 4;
-        const uint32_t old = atomicAdd(&hist[sx(b >> 1)], 1u << h);
-        bs[j] = (b << 10) | ((old >> h) & 0x3FFu);
-      }
-    }
-  }
-  __syncwarp();
-  // exclusive scan of the bucket counts; lane l owns counter words
-  // 32l..32l+31 (buckets 32l.. narrow, 64l.. wide)
-  uint32_t bigw = 0;  // bit k: a bucket of count word k holds 16 or more points
-  uint32_t rounds;    // transposition rounds the small buckets need
-  {
-    // two passes over the lane's row (the counts, then the starts), so that
-    // only one quad of it is held beside key and bs
-    uint32_t tot = 0, mx2 = 0;
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const uint4 t = *reinterpret_cast<const uint4 *>(hist + qoff(lane, m));
-      const uint32_t w4[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if constexpr (kNarrow) {
-          if (w4[e] >= (uint32_t)kEncSmall) bigw |= 1u << (4 * m + e);
-          tot += w4[e];
-          mx2 = max(mx2, w4[e]);
-        } else {
-          if (w4[e] & 0xFFF0FFF0u) bigw |= 1u << (4 * m + e);
-          tot += (w4[e] & 0xFFFFu) + (w4[e] >> 16);
-          mx2 = __vmaxu2(mx2, w4[e]);
-        }
-      }
-    }
-    if (kNarrow && __any_sync(FULL, bigw != 0u)) return false;
-    // a bucket of n points is in order after n alternating odd / even steps
-    // (whichever comes first), ceil(n / 2) rounds of the pair; buckets of 16
-    // or more are sorted already, so 8 rounds cover the rest
-    rounds = min((warp_max(max(mx2 & 0xFFFFu, mx2 >> 16)) + 1u) >> 1, (uint32_t)kEncSmall / 2u);
-    uint32_t inc = tot;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(FULL, inc, o);
-      if (lane >= o) inc += t;
-    }
-    uint32_t run = inc - tot;
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      uint4 *const q4 = reinterpret_cast<uint4 *>(hist + qoff(lane, m));
-      const uint4 t = *q4;
-      uint32_t w4[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if constexpr (kNarrow) {
-          const uint32_t c0 = w4[e];
-          w4[e] = run;
-          run += c0;
-        } else {
-          const uint32_t c0 = w4[e] & 0xFFFFu, c1 = w4[e] >> 16;
-          w4[e] = run | ((run + c0) << 16);
-          run += c0 + c1;
-        }
-      }
-      *q4 = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-    }
-  }
-  __syncwarp();
-  // place: bucket start + arrival slot; every point now lies inside its
-  // bucket's range of S, and the buckets are in order
-#pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    if (full || 32u * j + lane < nvalid) {
-      if constexpr (kNarrow) {
-        S[sx(hist[bs[j] >> 10] + (bs[j] & 0x3FFu))] = key[j];
-      } else {
-        const uint32_t b = bs[j] >> 10;
-        const uint32_t pos = ((hist[sx(b >> 1)] >> ((b & 1u) << 4)) & 0xFFFFu) + (bs[j] & 0x3FFu);
-        S[sx(pos)] = key[j];
-        bs[j] = (pos << 11) | b;
-      }
-    }
-  }
-  __syncwarp();
-  // buckets of 16 or more points (wide composites only; narrow chunks with
-  // one were declined): the whole warp sorts each one
-  while (!kNarrow && __any_sync(FULL, bigw != 0)) {
-    const int src = __ffs((int)__ballot_sync(FULL, bigw != 0)) - 1;
-    const int k = __ffs((int)__shfl_sync(FULL, bigw, src)) - 1;
-    if (lane == src) bigw &= bigw - 1;
-#pragma unroll 1
-    for (uint32_t b = 64u * src + 2 * k; b < 64u * src + 2 * k + 2; ++b) {
-      const uint32_t st = bucket_start(hist, b, nvalid), en = bucket_start(hist, b + 1, nvalid);
-      if (en - st >= (uint32_t)kEncSmall) warp_bitonic_u32(S, st, en - st, lane);
-    }
-  }
-  __syncwarp();
-  if constexpr (!kNarrow) {
-    // the bucket of every position (the bucket starts are done with; a sort
-    // inside a big bucket keeps its positions' bucket)
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (full || 32u * j + lane < nvalid) hist[sx(bs[j] >> 11)] = bs[j] & 0x7FFu;
-    __syncwarp();
-  }
+// Sum of the entries of warps before `warp`, and of all.
+__device__ __forceinline__ uint32_t before4(const uint4 &t, int warp, uint32_t &all) {
+  all = t.x + t.y + t.z + t.w;
+  return (warp > 0 ? t.x : 0u) + (warp > 1 ? t.y : 0u) + (warp > 2 ? t.z : 0u);
+}
+__device__ __forceinline__ uint32_t max4(const uint4 &t) { return max(max(t.x, t.y), max(t.z, t.w)); }
 
-  // sorted order: this lane's positions 32l..32l+31
-  {
-    uint32_t bpos[32];  // wide: the bucket of each position
+// Point of rank r: r = (p % 32) * 32 + p / 32 swaps the two five-bit halves.
+__device__ __forceinline__ uint32_t point_of_rank(uint32_t r) { return ((r * 1025u) >> 5) & 1023u; }
+
+__device__ __forceinline__ uint32_t warp_inc_scan(uint32_t v, int lane) {
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const uint4 t = *reinterpret_cast<const uint4 *>(S + qoff(lane, m));
-      key[4 * m] = t.x; key[4 * m + 1] = t.y; key[4 * m + 2] = t.z; key[4 * m + 3] = t.w;
-      if constexpr (!kNarrow) {
-        const uint4 u = *reinterpret_cast<const uint4 *>(hist + qoff(lane, m));
-        bpos[4 * m] = u.x; bpos[4 * m + 1] = u.y; bpos[4 * m + 2] = u.z; bpos[4 * m + 3] = u.w;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, v, o);
+    if (lane >= o) v += t;
+  }
+  return v;
+}
+
+// Stable radix sort of the chunk by block id, for chunks the buckets do not
+// suit (few distinct ids, a crowded bucket, a short last chunk): least
+// significant digit first over the points in rank order, so equal ids keep
+// the order of their ranks.  A warp takes 256 consecutive elements, 32 at a
+// time; lanes of one digit find each other by match.any and the first of them
+// advances the warp's counter of that digit, so an element's place is the
+// digit's start (scan over digits, warps within a digit) plus its arrival
+// number.  ceil(bits / 9) passes.
+// byr: ids by rank (rx); cnt: 4 KB of counters; perm: two permutations of
+// 1024 ranks.  Begins and ends with a barrier; returns the sorted ranks.
+static __device__ __noinline__ const uint16_t *radix_rank(const uint32_t *byr, uint32_t *scr, uint16_t *perm,
+                                                          uint32_t *tot, uint32_t idbits) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t passes = max((idbits + 8u) / 9u, 1u);
+  const uint32_t dbits = max((idbits + passes - 1u) / passes, 1u), D = 1u << dbits;
+  uint16_t *const cnt = reinterpret_cast<uint16_t *>(scr);  // [digit][warp]
+  unsigned long long *const c8 = reinterpret_cast<unsigned long long *>(scr);
+  __syncthreads();  // the ids by rank are in place, the counters' words free
+#pragma unroll 1
+  for (uint32_t ps = 0; ps < passes; ++ps) {
+    const uint32_t shift = ps * dbits;
+    for (uint32_t i = t; i < D / 2u; i += kEncThreads) reinterpret_cast<uint4 *>(scr)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    const uint16_t *const from = perm + ((ps + 1u) & 1u) * kChunk;
+    uint16_t *const to = perm + (ps & 1u) * kChunk;
+    uint32_t dr[8], off[8];  // digit << 10 | rank; arrival number in the warp's digit
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const uint32_t i = 256u * warp + 32u * s + lane;
+      const uint32_t r = ps == 0 ? i : (uint32_t)from[i] & 1023u;
+      const uint32_t d = (byr[rx(r)] >> shift) & (D - 1u);
+      const uint32_t peers = __match_any_sync(FULL, d);
+      const uint32_t lower = __popc(peers & ((1u << lane) - 1u));
+      uint16_t *const cw = cnt + 4u * d + warp;
+      const uint32_t old = *cw;
+      __syncwarp();
+      if (lower == 0u) *cw = (uint16_t)(old + __popc(peers));
+      __syncwarp();
+      dr[s] = (d << 10) | r;
+      off[s] = old + lower;
+    }
+    __syncthreads();
+    // exclusive scan over (digit, warp): thread t owns digits per * t ..
+    const uint32_t per = max(D / kEncThreads, 1u);
+    uint32_t sum = 0;
+    if (t * per < D)
+      for (uint32_t i = 0; i < per; ++i) {
+        const unsigned long long v = c8[t * per + i];
+        const uint32_t a = (uint32_t)v, b = (uint32_t)(v >> 32);
+        sum += (a & 0xFFFFu) + (a >> 16) + (b & 0xFFFFu) + (b >> 16);
+      }
+    const uint32_t inc = warp_inc_scan(sum, lane);
+    if (lane == 31) tot[warp] = inc;
+    __syncthreads();
+    uint32_t all;
+    uint32_t run = before4(ld4(tot), warp, all) + inc - sum;
+    if (t * per < D)
+      for (uint32_t i = 0; i < per; ++i) {
+        const unsigned long long v = c8[t * per + i];
+        const uint32_t a = (uint32_t)v, b = (uint32_t)(v >> 32);
+        const uint32_t s1 = run + (a & 0xFFFFu), s2 = s1 + (a >> 16), s3 = s2 + (b & 0xFFFFu);
+        c8[t * per + i] = (unsigned long long)(run | (s1 << 16)) | ((unsigned long long)(s2 | (s3 << 16)) << 32);
+        run = s3 + (b >> 16);
+      }
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < 8; ++s) to[(uint32_t)cnt[4u * (dr[s] >> 10) + warp] + off[s]] = (uint16_t)(dr[s] & 1023u);
+    __syncthreads();
+  }
+  return perm + ((passes + 1u) & 1u) * kChunk;
+}
+
+// Ascending sort of the n <= 32 K distinct values a[0..n) by one warp, K a
+// lane (lane l: values K l ..): a bitonic network whose exchanges all put the
+// minimum at the lower index (the first step of each merge pairs i with
+// i ^ (k - 1)), padded with the largest value.  Partners in other lanes come
+// by shuffles: about 60 / 150 / 250 / 460 instructions for K = 1 / 2 / 4 / 8,
+// where the same network in shared memory took 2,000 for 256 values.
+template <int K>
+__device__ __forceinline__ void warp_sort_regs(uint32_t *a, uint32_t n, int lane) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  uint32_t v[K];
+#pragma unroll
+  for (int e = 0; e < K; ++e) v[e] = (uint32_t)(K * lane + e) < n ? a[K * lane + e] : FULL;
+#pragma unroll
+  for (int k = 2; k <= 32 * K; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      const bool mirror = j == (k >> 1);
+      if (j < K && k <= K) {  // both in this lane
+#pragma unroll
+        for (int e = 0; e < K; ++e) {
+          const int p = mirror ? e ^ (k - 1) : e ^ j;
+          if (e < p) {
+            const uint32_t x = v[e], y = v[p];
+            v[e] = min(x, y);
+            v[p] = max(x, y);
+          }
+        }
+      } else if (j < K) {  // past a merge's first step, inside the lane
+#pragma unroll
+        for (int e = 0; e < K; ++e)
+          if ((e & j) == 0) {
+            const uint32_t x = v[e], y = v[e | j];
+            v[e] = min(x, y);
+            v[e | j] = max(x, y);
+          }
+      } else {
+        const int m = mirror ? k / K - 1 : j / K;  // partner lane ^ m
+        const bool upper = (lane & (j / K)) != 0;
+        uint32_t o[K];
+#pragma unroll
+        for (int e = 0; e < K; ++e) o[e] = __shfl_xor_sync(FULL, v[mirror ? K - 1 - e : e], m);
+#pragma unroll
+        for (int e = 0; e < K; ++e) v[e] = upper ? max(v[e], o[e]) : min(v[e], o[e]);
       }
     }
-    // positions past the chunk's end (stale words; the caller gives them the
-    // last id) take the largest value (narrow) or distinct out-of-range
-    // buckets (wide), so no step moves them
-    if (!full) {
+  }
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (32u * lane + j >= nvalid) {
-          if constexpr (kNarrow) key[j] = 0xFFFFFFFFu;
-          else bpos[j] = 0x80000000u | (32u * lane + j);
-        }
+  for (int e = 0; e < K; ++e)
+    if ((uint32_t)(K * lane + e) < n) a[K * lane + e] = v[e];
+}
+
+static __device__ __noinline__ void warp_sort_small(uint32_t *a, uint32_t n, int lane) {
+  if (n <= 32u) warp_sort_regs<1>(a, n, lane);
+  else if (n <= 64u) warp_sort_regs<2>(a, n, lane);
+  else if (n <= 128u) warp_sort_regs<4>(a, n, lane);
+  else warp_sort_regs<8>(a, n, lane);
+}
+
+// A chunk's points in registers, one 16-byte load (kVec points) at a time:
+// thread t's point e = kVec h + i is point 128 kVec h + kVec t + i of the
+// chunk.  Chunks of misaligned axes and a short last chunk load single points;
+// the latter's slots past the end hold a copy of its first point, which leaves
+// min / max, the id range and the relative positions' width unchanged.
+template <typename T>
+struct Points {
+  static constexpr int kVec = 16 / (int)sizeof(T);
+  __device__ __forceinline__ static uint32_t point(uint32_t t, int e) {
+    return 128u * kVec * (e / kVec) + kVec * t + (e % kVec);
+  }
+  // stable rank r(p) = (p % 32) * 32 + p / 32 of point(t, e): base(t) + step(e)
+  __device__ __forceinline__ static uint32_t rank_base(uint32_t t) {
+    return 32u * kVec * (t % (32 / kVec)) + t / (32 / kVec);
+  }
+  __host__ __device__ constexpr static uint32_t rank_step(int e) { return 32u * (e % kVec) + 4u * kVec * (e / kVec); }
+};
+
+// Ranks a full chunk's points through buckets over their id range.
+//  * kNarrow (ids below 2^22): 1024 buckets that split the range evenly
+//    (id * scale >> 32); S holds whole composites id << 10 | r.  H receives
+//    the sorted composites.
+//  * wide: buckets are the id bits from `low` up; S holds the bits below with
+//    r, and the bucket of every position lies beside (in Q).  H receives the
+//    sorted ids and Q the sorted ranks (16 bits each).
+// A few crowded buckets (kEncSmall points or more: a dense cluster) are sorted
+// by one warp each; with too many points in them (kEncCrowd, kEncCrowdPoints)
+// the result is false, S and H hold nothing of use and key is unchanged.  H
+// and sm.ncrowd must be clear; ends with a barrier.
+//
+// 32M clustered points with a few percent of them in one cluster: 0.85 ms when
+// any bucket of 16 points sent the chunk to the radix sort (three passes at
+// these id ranges), 0.41 ms so, 0.51 ms in the one-warp form.  Points in many
+// crowded buckets (ordered snapshots) are cheaper in the radix sort: hence the
+// second limit.
+template <typename T, bool kNarrow>
+__device__ __forceinline__ bool rank_buckets(EncShared &sm, uint32_t *H, uint32_t *S, const uint32_t (&key)[kEncPer],
+                                             uint32_t bound, int t, int lane, int warp) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  const uint32_t rbase = Points<T>::rank_base(t);
+  const uint32_t low = kNarrow ? 0u : 22u - __clz(bound);  // wide: id bits below the bucket
+  // 1024 * 2^32 / (bound + 1), a little less: id * scale >> 32 <= 1023
+  const uint32_t scale = kNarrow ? __float2uint_rz(__fdividef(4.39804e12f, __uint2float_rn(bound) + 1.0f)) : 0u;
+  uint32_t bs[kEncPer];  // arrival slot << 14 | bucket << 2
+#pragma unroll
+  for (int e = 0; e < kEncPer; ++e) {
+    // in range by construction; the mask keeps the access in bounds whatever the id
+    const uint32_t b = (kNarrow ? __umulhi(key[e], scale) : key[e] >> low) & (kEncBuckets - 1u);
+    bs[e] = (atomicAdd(&H[b], 1u) << 14) | (b << 2);
+  }
+  __syncthreads();  // counts
+  // exclusive scan; thread t owns buckets 8t..8t+7.  Starts are kept in bytes.
+  uint32_t c8[8];
+  {
+    const uint4 u0 = ld4(H + 8 * t), u1 = ld4(H + 8 * t + 4);
+    c8[0] = u0.x; c8[1] = u0.y; c8[2] = u0.z; c8[3] = u0.w;
+    c8[4] = u1.x; c8[5] = u1.y; c8[6] = u1.z; c8[7] = u1.w;
+  }
+  uint32_t sum = 0, mx = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    mx = max(mx, c8[i]);
+    const uint32_t n = c8[i];
+    c8[i] = sum;
+    sum += 4u * n;
+  }
+  const uint32_t inc = warp_inc_scan(sum, lane);
+  mx = warp_max(mx);
+  {
+    const uint32_t b0 = inc - sum;
+    *reinterpret_cast<uint4 *>(H + 8 * t) = make_uint4(c8[0] + b0, c8[1] + b0, c8[2] + b0, c8[3] + b0);
+    *reinterpret_cast<uint4 *>(H + 8 * t + 4) = make_uint4(c8[4] + b0, c8[5] + b0, c8[6] + b0, c8[7] + b0);
+  }
+  uint32_t pts = 0;
+  if (mx >= (uint32_t)kEncSmall) {  // the same for the whole warp
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t n = ((i < 7 ? c8[i < 7 ? i + 1 : 0] : sum) - c8[i]) >> 2;
+      if (n >= (uint32_t)kEncSmall) pts += n;
     }
-    // order inside the buckets of 2..15 points (they arrive in slot order;
-    // the big ones are sorted): odd-even transposition steps between
-    // neighbouring positions of one bucket, `rounds` pairs of steps
+    pts = __reduce_add_sync(FULL, pts);
+  }
+  if (lane == 31) {
+    sm.tot[warp] = inc;
+    sm.big[warp] = mx;
+    sm.cpts[warp] = pts;
+  }
+  __syncthreads();  // warps' totals
+  const uint32_t biggest = max4(ld4(sm.big));
+  // starts are relative to the quarter of the buckets a warp scanned
+  const uint4 tt = ld4(sm.tot);
+  const uint32_t q1 = tt.x, q2 = tt.x + tt.y, q3 = q2 + tt.z;
+  if (biggest >= (uint32_t)kEncSmall) {
+    const uint4 c4 = ld4(sm.cpts);
+    if (biggest > (uint32_t)kEncCrowd || c4.x + c4.y + c4.z + c4.w > (uint32_t)kEncCrowdPoints) return false;
+    const uint32_t b0 = inc - sum + (warp < 2 ? (warp == 0 ? 0u : q1) : (warp == 2 ? q2 : q3));
+    uint32_t ms = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t n = ((i < 7 ? c8[i < 7 ? i + 1 : 0] : sum) - c8[i]) >> 2;
+      if (n >= (uint32_t)kEncSmall) sm.crowd[atomicAdd(&sm.ncrowd, 1u)] = ((c8[i] + b0) << 14) | n;
+      else ms = max(ms, n);
+    }
+    ms = warp_max(ms);
+    if (lane == 0) sm.small[warp] = ms;
+  }
+  uint16_t *const Bk = reinterpret_cast<uint16_t *>(sm.Q);
+  const uint32_t lmask = (1u << low) - 1u;
+#pragma unroll
+  for (int e = 0; e < kEncPer; ++e) {
+    const uint32_t b4 = bs[e] & 0xFFCu;
+    const uint32_t quarter = b4 < 2048u ? (b4 < 1024u ? 0u : q1) : (b4 < 3072u ? q2 : q3);
+    const uint32_t pos4 = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(H) + b4) + (bs[e] >> 12) + quarter;
+    const uint32_t v = ((kNarrow ? key[e] : key[e] & lmask) << 10) + (rbase + Points<T>::rank_step(e));
+    *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(S) + pos4) = v;
+    if (!kNarrow) Bk[pos4 >> 2] = (uint16_t)(b4 >> 2);
+  }
+  __syncthreads();  // placed
+  uint32_t largest = biggest;  // of the buckets still to order
+  if (biggest >= (uint32_t)kEncSmall) {
+    for (uint32_t k = warp; k < sm.ncrowd; k += kEncWarps) warp_sort_small(S + (sm.crowd[k] >> 16), sm.crowd[k] & 0xFFFFu, lane);
+    largest = max4(ld4(sm.small));
+    __syncthreads();  // crowded buckets in order
+  }
+  // Order inside the buckets: every warp takes its 256 positions and 16 more
+  // on either side (32 on one side at the chunk's ends), nine a lane; such a
+  // bucket has at most 15 points, so each of the warp's own positions sees its
+  // whole bucket.  Neighbours are compared
+  // in the order even pairs, across lanes, odd pairs, across lanes: ceil(n / 2)
+  // rounds order a bucket of n points wherever it lies.
+  uint32_t k9[kEncOrd];
+  const uint32_t w0 = warp == 0 ? 0u : (warp == kEncWarps - 1 ? kChunk - 32u * kEncOrd : 256u * warp - kEncHalo);
+  const uint32_t p0 = w0 + kEncOrd * lane, o0 = p0 - 256u * warp;
+#pragma unroll
+  for (int j = 0; j < kEncOrd; ++j) k9[j] = S[p0 + j];
+  const uint32_t rounds = (largest + 1u) >> 1;
+  if (kNarrow) {
+    // neighbours of different buckets are in order already
 #pragma unroll 1
     for (uint32_t it = 0; it < rounds; ++it) {
 #pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const bool x = (kNarrow || bpos[j] == bpos[j + 1]) && key[j] > key[j + 1];
-        const uint32_t lo = x ? key[j + 1] : key[j], hi = x ? key[j] : key[j + 1];
-        key[j] = lo; key[j + 1] = hi;
-      }
-      const uint32_t nk = __shfl_down_sync(FULL, key[0], 1), pk = __shfl_up_sync(FULL, key[31], 1);
-      const uint32_t nb = kNarrow ? 0u : __shfl_down_sync(FULL, bpos[0], 1);
-      const uint32_t pb = kNarrow ? 0u : __shfl_up_sync(FULL, bpos[31], 1);
+      for (int h = 0; h < 2; ++h) {
 #pragma unroll
-      for (int j = 1; j < 31; j += 2) {
-        const bool x = (kNarrow || bpos[j] == bpos[j + 1]) && key[j] > key[j + 1];
-        const uint32_t lo = x ? key[j + 1] : key[j], hi = x ? key[j] : key[j + 1];
-        key[j] = lo; key[j + 1] = hi;
+        for (int j = h; j + 1 < kEncOrd; j += 2) {
+          const uint32_t x = k9[j], y = k9[j + 1];
+          k9[j] = min(x, y);
+          k9[j + 1] = max(x, y);
+        }
+        const uint32_t nx = __shfl_down_sync(FULL, k9[0], 1), pv = __shfl_up_sync(FULL, k9[kEncOrd - 1], 1);
+        if (lane < 31) k9[kEncOrd - 1] = min(k9[kEncOrd - 1], nx);
+        if (lane > 0) k9[0] = max(k9[0], pv);
       }
-      // the pair across lanes: positions 32l+31 and 32(l+1); both lanes
-      // decide on the same two values
-      const bool xr = lane < 31 && (kNarrow || nb == bpos[31]) && key[31] > nk;
-      const bool xl = lane > 0 && (kNarrow || pb == bpos[0]) && pk > key[0];
-      if (xr) key[31] = nk;
-      if (xl) key[0] = pk;
     }
 #pragma unroll
-    for (int k = 0; k < 16; ++k) rp[k] = (key[k] & 1023u) | ((key[k + 16] & 1023u) << 16);
+    for (int j = 0; j < kEncOrd; ++j)
+      if (o0 + j < 256u) H[p0 + j] = k9[j];
+  } else {
+    // cut[j] = all ones where positions j and j+1 are of different buckets
+    // (never exchanged), the last entry towards the next lane
+    uint32_t b9[kEncOrd], cut[kEncOrd];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      if constexpr (kNarrow) key[j] = kmin + (key[j] >> 10);
-      else key[j] = kmin + ((bpos[j] << lowb) | (key[j] >> 10));
+    for (int j = 0; j < kEncOrd; ++j)
+      b9[j] = (uint32_t)Bk[p0 + j];
+    const uint32_t nb = __shfl_down_sync(FULL, b9[0], 1);
+#pragma unroll
+    for (int j = 0; j + 1 < kEncOrd; ++j) cut[j] = b9[j] == b9[j + 1] ? 0u : FULL;
+    cut[kEncOrd - 1] = lane < 31 && b9[kEncOrd - 1] == nb ? 0u : FULL;
+    uint32_t pcut = __shfl_up_sync(FULL, cut[kEncOrd - 1], 1);
+    if (lane == 0) pcut = FULL;
+    __syncthreads();  // the buckets have been read: Q takes the ranks
+#pragma unroll 1
+    for (uint32_t it = 0; it < rounds; ++it) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int j = h; j + 1 < kEncOrd; j += 2) {
+          const uint32_t x = k9[j], y = k9[j + 1];
+          k9[j] = min(x, y | cut[j]);
+          k9[j + 1] = max(x & ~cut[j], y);
+        }
+        const uint32_t nx = __shfl_down_sync(FULL, k9[0], 1), pv = __shfl_up_sync(FULL, k9[kEncOrd - 1], 1);
+        k9[kEncOrd - 1] = min(k9[kEncOrd - 1], nx | cut[kEncOrd - 1]);
+        k9[0] = max(k9[0], pv & ~pcut);
+      }
     }
+#pragma unroll
+    for (int j = 0; j < kEncOrd; ++j)
+      if (o0 + j < 256u) {
+        H[p0 + j] = (b9[j] << low) | (k9[j] >> 10);
+        Bk[p0 + j] = (uint16_t)(k9[j] & 1023u);
+      }
   }
-  __syncwarp();
-#pragma unroll
-  for (int m = 0; m < 8; ++m)
-    *reinterpret_cast<uint4 *>(S + qoff(lane, m)) = make_uint4(key[4 * m], key[4 * m + 1], key[4 * m + 2], key[4 * m + 3]);
-#pragma unroll
-  for (int m = 0; m < 4; ++m)
-    *reinterpret_cast<uint4 *>(hist + qoff(lane, m)) = make_uint4(rp[4 * m], rp[4 * m + 1], rp[4 * m + 2], rp[4 * m + 3]);
-  __syncwarp();
+  __syncthreads();  // ranked
   return true;
 }
 
-// A quantized chunk between the two encode phases: its 31-bit block ids
-// (element j of lane l is point 32j + l), their range, the relative-position
-// bit width and this lane's word of the meta record's min/max part.
-struct ChunkQ {
-  uint32_t key[32];
-  uint32_t kmin, kmax, rbits, mword;
-};
-
-// The points of one chunk, loaded ahead of encoding: float streams keep all
-// axes in registers (element j of lane l is point 32j + l of the chunk), so a
-// chunk costs one round of loads and the next chunk's loads overlap the
-// current one's placement.  Double streams load one axis at a time.
-//
-// The slots past the end of a short last chunk hold a copy of the chunk's
-// first point: they leave the chunk's min / max, id range and largest
-// relative position unchanged, so the encoder's per-point loops need no
-// validity test and only the ranking and the relative-position section treat
-// those slots specially.
 template <typename T, int DIM>
-struct ChunkPoints {
-  static constexpr bool kAhead = sizeof(T) == 4;
-  T v[kAhead ? DIM : 1][32];
-  __device__ __forceinline__ void load(const CArgs<T> &a, unsigned long long c, int lane) {
-    if constexpr (kAhead) {
-      c = c < a.G ? c : a.G - 1;  // past the end: reload the last chunk (unused)
-      const unsigned long long base = c * kChunk;
-      const uint32_t nvalid = (uint32_t)min((unsigned long long)kChunk, a.n - base);
-      const T *const X[3] = {a.x, a.y, a.z};
-      if (nvalid == (uint32_t)kChunk) {
+__device__ __forceinline__ void load_points(const CArgs<T> &a, unsigned long long base, uint32_t nvalid,
+                                            T (&v)[DIM][kEncPer]) {
+  constexpr int V = Points<T>::kVec;
+  const uint32_t t = threadIdx.x;
+  const T *const X[3] = {a.x + base, a.y + base, a.z + base};
+  uint32_t low = (uint32_t)(uintptr_t)a.x | (uint32_t)(uintptr_t)a.y;
+  if (DIM == 3) low |= (uint32_t)(uintptr_t)a.z;
+  if (nvalid == (uint32_t)kChunk && (low & 15u) == 0u) {
 #pragma unroll
-        for (int d = 0; d < DIM; ++d)
+    for (int d = 0; d < DIM; ++d)
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[d][j] = X[d][base + 32u * j + lane];
-      } else {
-#pragma unroll
-        for (int d = 0; d < DIM; ++d)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const uint32_t p = 32u * j + lane;
-            v[d][j] = X[d][base + (p < nvalid ? p : 0u)];
-          }
-      }
-    } else {
-      // Double streams keep no points in registers: lane d asks for axis d
-      // of the chunk in L2 (one bulk prefetch of its valid, 16-byte aligned
-      // span), so that the quantize phase's loads hit L2.
-      if (lane < DIM && c < a.G) {
-        const unsigned long long base = c * kChunk;
-        const uint32_t nvalid = (uint32_t)min((unsigned long long)kChunk, a.n - base);
-        const T *p = (lane == 0 ? a.x : (lane == 1 ? a.y : a.z)) + base;
-        const uint32_t bytes = (nvalid * (uint32_t)sizeof(T)) & ~15u;
-        if (bytes != 0u && (reinterpret_cast<uintptr_t>(p) & 15u) == 0u)
-          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-      }
-    }
-  }
-};
-
-// First phase of encoding chunk c: min/max, quantization, block ids (into q)
-// and relative positions (into the warp's third 4 KB, by rank r); double
-// streams also stage each axis in the region's first 8 KB.
-template <typename T, int DIM>
-__device__ __forceinline__ void encode_quantize(const CArgs<T> &a, unsigned long long c, uint32_t *sw,
-                                                uint32_t seg, uint32_t sh, uint32_t msk, T eb, T inv,
-                                                ChunkPoints<T, DIM> &pts, ChunkQ &q, int lane) {
-  using Tr = TT<T>;
-  using UO = typename Tr::U;
-  constexpr bool is64 = sizeof(T) == 8;
-  constexpr uint32_t FULL = 0xFFFFFFFFu;
-  const unsigned long long n = a.n;
-  const unsigned long long base = c * kChunk;
-  const uint32_t nvalid = (uint32_t)min((unsigned long long)kChunk, n - base);
-  const bool full = nvalid == (uint32_t)kChunk;
-  uint32_t *const relR = sw + 2 * kChunk;
-  const T *const X[3] = {a.x, a.y, a.z};
-
-  // ---- 1. quantize one axis at a time (:104-205) ----
-  uint32_t (&key)[32] = q.key;
-  T mm[6];
-  unsigned long long bnx = 0, bny = 0, bound = 0;
-  uint32_t rmax = 0;
-  // Double streams stage each axis in the warp's first 8 KB (free while a
-  // chunk is quantized: the previous payload has been copied out), element j
-  // of lane l at word pair 32j + l, so the min/max and quantize passes read
-  // it back without holding 32 doubles in registers.
-  T *const stash = reinterpret_cast<T *>(sw);
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) {
-    if constexpr (!ChunkPoints<T, DIM>::kAhead) {
-      const T *src = X[d] + base;
-      if (d > 0) __syncwarp();  // the previous axis has been read
-      if (full && a.vec_ok) {
-        // a full chunk of 16-byte aligned axes: 16-byte asynchronous copies,
-        // 16 per lane, all in flight at once, no registers
-        const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(stash) + 16u * lane;
-        const char *g0 = reinterpret_cast<const char *>(src) + 16u * lane;
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s0 + 512u * i), "l"(g0 + 512u * i) : "memory");
-        asm volatile("cp.async.wait_all;" ::: "memory");
-      } else {
-#pragma unroll 8
-        for (int j = 0; j < 32; ++j) {
-          const uint32_t p = 32u * j + lane;
-          stash[p] = (full || p < nvalid) ? src[p] : src[0];  // past the end: the first point
-        }
-      }
-      __syncwarp();
-    }
-    auto vv_of = [&](int j) -> T {
-      if constexpr (ChunkPoints<T, DIM>::kAhead) return pts.v[d][j];
-      else return stash[32u * j + lane];
-    };
-    // fmin / fmax ignore NaN and order -0.0 below +0.0, as the reference's
-    // warp reductions do (:122-139); slots past the end repeat a point
-    const T lim = is64 ? (T)DBL_MAX : (T)FLT_MAX;
-    T mn = lim, mx = -lim;
-    if constexpr (!is64) {
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        mn = fmin3f(mn, vv_of(j), vv_of(j + 1));
-        mx = fmax3f(mx, vv_of(j), vv_of(j + 1));
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) { mn = fmin(mn, vv_of(j)); mx = fmax(mx, vv_of(j)); }
-    }
-    mn = from_ord((UO)~warp_max((UO)~ord_of(mn)));
-    mx = from_ord(warp_max(ord_of(mx)));
-    mm[d] = mn;
-    mm[3 + d] = mx;
-    const T range = is64 ? (T)__dsub_rn((double)mx, (double)mn) : (T)__fsub_rn((float)mx, (float)mn);
-    if (d == 0) bnx = block_num(range, seg, eb, is64 && DIM == 2);
-    if (d == 1) bny = block_num(range, seg, eb, false);
-    const T nmn = is64 ? (T)__dmul_rn(-(double)mn, (double)inv) : (T)__fmul_rn(-(float)mn, (float)inv);
-    // id_overflow: the chunk's largest quantized corner (u64 arithmetic)
-    const unsigned long long qm = is64 ? __double2ull_rz(__fma_rn((double)mx, (double)inv, (double)nmn))
-                                       : (unsigned long long)__float2uint_rz(__fmaf_rn((float)mx, (float)inv, (float)nmn));
-    bound += (qm >> sh) * (d == 0 ? 1ull : (d == 1 ? bnx : bnx * bny));
-    // block id (mod 2^32, masked to 31 bits at the end) and relative position
-    const uint32_t kmul = d == 0 ? 1u : (d == 1 ? (uint32_t)bnx : (uint32_t)(bnx * bny));
-    const uint32_t rmul = d == 0 ? 1u : (d == 1 ? seg : seg * seg);
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      uint32_t rq[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int j = 4 * m + e;
-        uint32_t kq, r;
-        if constexpr (!is64) {
-          const uint32_t q = __float2uint_rz(__fmaf_rn((float)vv_of(j), (float)inv, (float)nmn));
-          kq = q >> sh;
-          r = q & msk;
+      for (int h = 0; h < kEncPer / V; ++h) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(X[d]) + 128 * h + t);
+        if constexpr (sizeof(T) == 4) {
+          v[d][4 * h] = __uint_as_float(q.x); v[d][4 * h + 1] = __uint_as_float(q.y);
+          v[d][4 * h + 2] = __uint_as_float(q.z); v[d][4 * h + 3] = __uint_as_float(q.w);
         } else {
-          const unsigned long long q = __double2ull_rz(__fma_rn((double)vv_of(j), (double)inv, (double)nmn));
-          kq = (uint32_t)(q >> sh);
-          r = (uint32_t)(q & msk);
-        }
-        key[j] = d == 0 ? kq : key[j] + kq * kmul;
-        rq[e] = r * rmul;
-      }
-      uint4 *row = reinterpret_cast<uint4 *>(relR + qoff(lane, m));
-      if (d > 0) {
-        const uint4 o = *row;
-        rq[0] += o.x; rq[1] += o.y; rq[2] += o.z; rq[3] += o.w;
-      }
-      if (d == DIM - 1) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          rq[e] &= 0x7FFFFFFFu;
-          rmax = max(rmax, rq[e]);
+          v[d][2 * h] = __hiloint2double((int)q.y, (int)q.x);
+          v[d][2 * h + 1] = __hiloint2double((int)q.w, (int)q.z);
         }
       }
-      *row = make_uint4(rq[0], rq[1], rq[2], rq[3]);
-    }
-  }
-  if (DIM == 2) { mm[2] = (T)0; mm[5] = (T)0; }  // 2D meta carries z = 0 (:518, :521)
-  // this lane's word of the meta record's min/max part (:332-344 / Double
-  // :333-345), taken now so the six values need no registers later
-  uint32_t mword = 0;
-  {
-    T mv = mm[0];
+  } else {
 #pragma unroll
-    for (int k = 1; k < 6; ++k)
-      if ((is64 ? (lane >> 1) : lane) == k) mv = mm[k];
-    if (!is64) {
-      mword = __float_as_uint((float)mv);
-    } else {
-      const unsigned long long b = (unsigned long long)__double_as_longlong((double)mv);
-      mword = (lane & 1) ? (uint32_t)(b >> 32) : (uint32_t)b;
-    }
-  }
-  if (lane == 0 && bound > 0x7FFFFFFFull) a.ctl->id_overflow = 1u;
-  uint32_t kmin = FULL, kmax = 0;
+    for (int d = 0; d < DIM; ++d)
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    key[j] &= 0x7FFFFFFFu;
-    kmin = min(kmin, key[j]);
-    kmax = max(kmax, key[j]);
+      for (int e = 0; e < kEncPer; ++e) {
+        const uint32_t p = Points<T>::point(t, e);
+        v[d][e] = __ldg(X[d] + (p < nvalid ? p : 0u));
+      }
   }
-  q.kmin = warp_min(kmin);
-  q.kmax = warp_max(kmax);
-  rmax = warp_max(rmax);
-  q.rbits = max(bitlen(rmax), nvalid < (uint32_t)kChunk ? 1u : 0u);  // :200-201
-  q.mword = mword;
 }
 
-// Ranks, runs and bit planes of a quantized chunk (encode_quantize left its
-// ids in q and its relative positions in the warp's third 4 KB); stages the
-// payload in the warp's region, returns its bytes and leaves the meta record
-// in meta_word (word k of the record in lane k).
-template <typename T, int DIM, class OnSize>
-__device__ __forceinline__ uint32_t encode_pack(const CArgs<T> &a, unsigned long long c, uint32_t *sw, ChunkQ &q,
-                                                uint32_t &meta_word, int lane, uint32_t &rank_skip,
-                                                OnSize &&on_size) {
+// Asks for chunk c's axes in L2 (bulk prefetches of the 16-byte aligned
+// spans, one lane per axis), ahead of its load.
+template <typename T, int DIM>
+__device__ __forceinline__ void prefetch_points(const CArgs<T> &a, unsigned long long c, int lane) {
+  if (lane < DIM && c < a.G) {
+    const unsigned long long base = c * kChunk;
+    const uint32_t nvalid = (uint32_t)min((unsigned long long)kChunk, a.n - base);
+    const T *p = (lane == 0 ? a.x : (lane == 1 ? a.y : a.z)) + base;
+    const uint32_t bytes = (nvalid * (uint32_t)sizeof(T)) & ~15u;
+    if (bytes != 0u && (reinterpret_cast<uintptr_t>(p) & 15u) == 0u)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+  }
+}
+
+// The parked payloads of a CTA: `count` of them, the oldest in slot `head`.
+struct Parked {
+  uint32_t head, count;
+};
+
+// Header of the stream (:1674-1678; Double :1672-1680), by the first warp.
+template <typename T>
+__device__ __forceinline__ void put_header(const CArgs<T> &a, T eb, uint32_t seg, int lane) {
+  uint32_t *h = reinterpret_cast<uint32_t *>(a.out);
+  if (lane == 0) h[0] = a.dim;
+  if (lane == 1) h[1] = (uint32_t)a.n;
+  if (lane == 2) h[2] = (uint32_t)(a.n >> 32);
+  if (lane == 3) h[3] = TT<T>::bits;
+  if constexpr (sizeof(T) == 4) {
+    if (lane == 4) h[4] = __float_as_uint((float)eb);
+    if (lane == 5) h[5] = seg;
+  } else {
+    if (lane == 4) h[4] = (uint32_t)__double_as_longlong((double)eb);
+    if (lane == 5) h[5] = (uint32_t)((unsigned long long)__double_as_longlong((double)eb) >> 32);
+    if (lane == 6) h[6] = seg;
+    if (lane == 7) h[7] = 32u;
+  }
+}
+
+// Places the payload in `slot` at stream offset sm.goff, with its offset-table
+// entry (:1679), and sets the stream's size after the last chunk.
+template <typename T>
+__device__ __forceinline__ void place_parked(const CArgs<T> &a, EncShared &sm, uint32_t slot) {
+  using Tr = TT<T>;
+  const unsigned long long off = sm.goff, c = sm.park[slot].c;
+  const uint32_t payload = sm.park[slot].payload;
+  if (off >= kGoffPending) return;  // the look-back gave up
+  const uint32_t *const P = sm.P[slot];
+  const unsigned long long G = a.G, pay_base = Tr::hdr + 8ull * G + (unsigned long long)Tr::meta * G;
+  const int t = (int)threadIdx.x;
+  constexpr int N = kEncThreads;
+  if (t == 0) reinterpret_cast<unsigned long long *>(a.out + Tr::hdr)[c] = off;
+  if (pay_base + off + payload > a.out_cap) {
+    if (t == 0) set_status(a.ctl, kENOSPACE);
+  } else {
+    // four words in flight per thread: one shared-memory latency per 1.5 KB
+    uint32_t *const dst = reinterpret_cast<uint32_t *>(a.out + pay_base + off);
+    const uint32_t nw = payload / 4u;
+    uint32_t w = t;
+    for (; w + 3 * N < nw; w += 4 * N) {
+      uint32_t v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = P[w + i * N];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dst[w + i * N] = v[i];
+    }
+    for (; w < nw; w += N) dst[w] = P[w];
+  }
+  if (c == G - 1 && t == 0) a.ctl->stream_bytes = pay_base + off + payload;
+}
+
+// One warp: the stream offset of the payload in `slot` into sm.goff (kGoffPending when
+// a predecessor's size is missing and `wait` is not set).
+template <typename T>
+__device__ __forceinline__ void look_up(const CArgs<T> &a, uint32_t slot, EncShared &sm, bool wait, int lane) {
+  unsigned long long excl = 0;
+  const int ok = resolve_prefix(a.ctl, a.look, sm.park[slot].c, excl, wait ? kSpinLimit : 0u, wait);
+  if (lane == 0) sm.goff = ok > 0 ? excl : (ok < 0 ? kGoffPending : kGoffNone);
+}
+
+// The chunk's scalars, by the first warp: per-axis values in lanes 0..2 (lane
+// d: axis d).  Block counts, id multipliers, offsets -min / (2 eb), the
+// largest block id, the meta record's min / max (:332-344 / Double :333-345).
+template <typename T, int DIM>
+__device__ __forceinline__ void chunk_scalars(const CArgs<T> &a, unsigned long long c, EncShared &sm, uint32_t seg,
+                                              uint32_t sh, T eb, T inv, int lane) {
   using Tr = TT<T>;
   constexpr bool is64 = sizeof(T) == 8;
   constexpr uint32_t FULL = 0xFFFFFFFFu;
+  T mmv;
+  {
+    const int k = lane < 6 ? (lane < 3 ? lane : lane + 1) : 0;
+    T v[kEncWarps];
+#pragma unroll
+    for (int i = 0; i < kEncWarps; ++i) v[i] = reinterpret_cast<const T *>(sm.mm[i])[k];
+    static_assert(kEncWarps == 4, "");
+    const T lo = min2(min2(v[0], v[1]), min2(v[2], v[3]));
+    const T hi = max2(max2(v[0], v[1]), max2(v[2], v[3]));
+    mmv = lane < 3 ? lo : hi;
+    if (DIM == 2 && (lane == 2 || lane == 5)) mmv = (T)0;  // 2D meta carries z = 0 (:518, :521)
+  }
+  const T mxv = __shfl_down_sync(FULL, mmv, 3);
+  const T range = is64 ? (T)__dsub_rn((double)mxv, (double)mmv) : (T)__fsub_rn((float)mxv, (float)mmv);
+  unsigned long long bn = block_num(range, seg, eb, false);
+  if (is64 && DIM == 2) {
+    const unsigned long long bw = block_num(range, seg, eb, true);
+    bn = lane == 0 ? bw : bn;
+  }
+  const T nm = is64 ? (T)__dmul_rn(-(double)mmv, (double)inv) : (T)__fmul_rn(-(float)mmv, (float)inv);
+  const unsigned long long qm = is64 ? __double2ull_rz(__fma_rn((double)mxv, (double)inv, (double)nm))
+                                     : (unsigned long long)__float2uint_rz(__fmaf_rn((float)mxv, (float)inv, (float)nm));
+  unsigned long long bnx, bny;
+  if (is64) {
+    bnx = __shfl_sync(FULL, bn, 0);
+    bny = __shfl_sync(FULL, bn, 1);
+  } else {
+    bnx = __shfl_sync(FULL, (uint32_t)bn, 0);
+    bny = __shfl_sync(FULL, (uint32_t)bn, 1);
+  }
+  const unsigned long long mult = lane == 0 ? 1ull : (lane == 1 ? bnx : bnx * bny);
+  const unsigned long long term = lane < DIM ? (qm >> sh) * mult : 0ull;
+  // the chunk's largest quantized corner: every quantized value is at most its
+  // axis's (the multiply-add and the truncation are monotone), so no id is
+  // above the sum; ids are masked to 31 bits when it does not fit
+  const float tf = lane < DIM ? __ull2float_rn(qm >> sh) * __ull2float_rn(mult) : 0.0f;
+  const bool wide = __any_sync(FULL, tf >= 7.0e8f);
+  const uint32_t sum = __reduce_add_sync(FULL, (uint32_t)term);
+  if (lane < 3) reinterpret_cast<T *>(sm.nm)[lane] = nm;
+  if (lane == 0) *reinterpret_cast<uint4 *>(sm.sc) = make_uint4((uint32_t)bnx, (uint32_t)(bnx * bny), wide ? 0x7FFFFFFFu : sum, 0u);
+  if (wide) {
+    // id_overflow: the same corner in u64 arithmetic (terms below 7e8 cannot
+    // reach 2^31).  Set once per CTA and stream: the flag shares its cache line
+    // with the work counter, and a store per chunk took 50M double points from
+    // 1.1 to 2.3 ms.
+    const unsigned long long corner = term + __shfl_down_sync(FULL, term, 1) + __shfl_down_sync(FULL, term, 2);
+    if (lane == 0 && corner > 0x7FFFFFFFull && sm.overflowed != a.ctl) {
+      a.ctl->id_overflow = 1u;
+      sm.overflowed = a.ctl;
+    }
+  }
+  uint8_t *meta = a.out + Tr::hdr + 8ull * a.G + (unsigned long long)Tr::meta * c;
+  if (lane < 6) reinterpret_cast<T *>(meta)[lane] = mmv;
+  if (c == 0) put_header<T>(a, eb, seg, lane);
+}
+
+// Encodes chunk c into a free slot of sm.P (see the top of the file) and
+// returns it.  `par` is the iteration's parity, pa[slot] the arguments of a
+// parked chunk; `claim` and, a phase later, `commit` run on the third warp (the
+// next chunk is claimed and its points prefetched).  rank_skip counts the
+// chunks still to sort without trying the buckets, declined the chunks the
+// buckets have declined in a row.
+template <typename T, int DIM, class PArgs, class Claim, class Commit>
+__device__ __forceinline__ uint32_t encode_chunk(const CArgs<T> &a, unsigned long long c, EncShared &sm, int par,
+                                                 uint32_t seg, T eb, T inv, const PArgs &pa, Parked &pk,
+                                                 uint32_t &rank_skip, uint32_t &declined, Claim &&claim, Commit &&commit) {
+  using Tr = TT<T>;
+  constexpr bool is64 = sizeof(T) == 8;
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t sh = (uint32_t)__ffs((int)seg) - 1u, msk = seg - 1u;
   const unsigned long long base = c * kChunk;
   const uint32_t nvalid = (uint32_t)min((unsigned long long)kChunk, a.n - base);
   const bool full = nvalid == (uint32_t)kChunk;
-  // per-warp words: [0,1024) ranked composites -> run starts -> staged payload;
-  // [1024,2048) bucket counts -> deltas -> staged payload; [2048,3072)
-  // relative positions by rank r (staged payload only past 8 KB, after use)
-  uint32_t *const S = sw, *const hist = sw + kChunk, *const relR = sw + 2 * kChunk;
-  uint32_t (&key)[32] = q.key;
-  const uint32_t kmin = q.kmin, kmax = q.kmax, rbits = q.rbits, mword = q.mword;
+  uint32_t *const H = sm.A[par], *const S = sm.A[par ^ 1];
+  bool pending;  // the oldest payload has to leave before this chunk's planes
 
-  // ---- 2. rank the composites (block id - kmin) << 10 | r ----
-  const unsigned long long cmax = ((unsigned long long)(kmax - kmin) << 10) | 1023ull;
-  const uint32_t cbits_all = bitlen64(cmax);
-  uint32_t rp[16];  // rank r of positions j and j+16 (16-bit pairs)
-  // Buckets rank every chunk whose composites are wider than 32 bits, and
-  // the 32-bit ones of at least 21 bits unless they have a bucket of 16 or
-  // more points (then the chunk is declined and the warp sorts its next
-  // kEncBucketBackoff chunks directly); the data-independent warp sort ranks
-  // the rest.  Both give the same order.
-  bool ranked = false;
-  if (cbits_all > 32u || (cbits_all >= 21u && rank_skip == 0u)) {
-    // block ids in and results out through S and hist rows
+  // ---- 1. points, min / max, quantization (:104-205) ----
+  uint32_t key[kEncPer];
+  uint32_t bound;  // no block id is above it
+  {
+    T v[DIM][kEncPer];
+    load_points<T, DIM>(a, base, nvalid, v);
+    // bucket counts (last used as run starts, done with before the last chunk's planes)
+    *reinterpret_cast<uint4 *>(H + 8 * t) = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4 *>(H + 8 * t + 4) = make_uint4(0u, 0u, 0u, 0u);
+    if (t == 0) sm.ncrowd = 0u;
+    // NaNs are ignored and -0.0 orders below +0.0, as in the reference's warp
+    // reductions (:122-139); slots past the end repeat a point
+    T mn[3], mx[3];
 #pragma unroll
-    for (int m = 0; m < 8; ++m)
-      *reinterpret_cast<uint4 *>(S + qoff(lane, m)) = make_uint4(key[4 * m], key[4 * m + 1], key[4 * m + 2], key[4 * m + 3]);
-    ranked = cbits_all > 32u ? rank_buckets<false>(sw, kmin, cbits_all, nvalid, lane)
-                             : rank_buckets<true>(sw, kmin, cbits_all, nvalid, lane);
+    for (int d = 0; d < DIM; ++d) warp_minmax(v[d], mn[d], mx[d]);
+    if (lane == 0) {
+      T *const m = reinterpret_cast<T *>(sm.mm[warp]);
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const uint4 t = *reinterpret_cast<const uint4 *>(S + qoff(lane, m));
-      key[4 * m] = t.x; key[4 * m + 1] = t.y; key[4 * m + 2] = t.z; key[4 * m + 3] = t.w;
+      for (int d = 0; d < DIM; ++d) {
+        m[d] = mn[d];
+        m[4 + d] = mx[d];
+      }
     }
-    if (ranked) {
-      if (!full) {  // positions past the end carry the last id: they start no run
+    __syncthreads();  // 1: minima and maxima, the oldest parked payload's offset
+    pending = pk.count == (uint32_t)kEncSlots;
+    if (warp == 0) chunk_scalars<T, DIM>(a, c, sm, seg, sh, eb, inv, lane);
+    else if (warp == kEncWarps - 1 && pending) look_up<T>(pa[pk.head], pk.head, sm, false, lane);
+    __syncthreads();  // 2: the chunk's scalars
+
+    // block id (mod 2^32, masked to 31 bits) and relative position
+    const uint4 sc = ld4(sm.sc);
+    bound = sc.z;
+    uint32_t rel[kEncPer];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) key[j] = 32u * lane + j < nvalid ? key[j] : kmax;
-      }
+    for (int d = 0; d < DIM; ++d) {
+      const T nmd = reinterpret_cast<const T *>(sm.nm)[d];
+      const uint32_t kmul = d == 1 ? sc.x : sc.y;
+      const uint32_t rmul = d == 1 ? seg : seg * seg;
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const uint4 t = *reinterpret_cast<const uint4 *>(hist + qoff(lane, m));
-        rp[4 * m] = t.x; rp[4 * m + 1] = t.y; rp[4 * m + 2] = t.z; rp[4 * m + 3] = t.w;
+      for (int e = 0; e < kEncPer; ++e) {
+        uint32_t kq, r;
+        if constexpr (!is64) {
+          const uint32_t q = __float2uint_rz(__fmaf_rn((float)v[d][e], (float)inv, (float)nmd));
+          kq = q >> sh;
+          r = q & msk;
+        } else {
+          const unsigned long long q = __double2ull_rz(__fma_rn((double)v[d][e], (double)inv, (double)nmd));
+          kq = (uint32_t)(q >> sh);
+          r = (uint32_t)q & msk;
+        }
+        key[e] = d == 0 ? kq : key[e] + kq * kmul;
+        rel[e] = d == 0 ? r : rel[e] + r * rmul;
       }
+    }
+    uint32_t orv = 0;
+#pragma unroll
+    for (int e = 0; e < kEncPer; ++e) {
+      key[e] &= 0x7FFFFFFFu;
+      rel[e] &= 0x7FFFFFFFu;
+      orv |= rel[e];
+    }
+    if constexpr (!is64) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<uint4 *>(sm.R + 512 * h + 4 * t) =
+            make_uint4(rel[4 * h], rel[4 * h + 1], rel[4 * h + 2], rel[4 * h + 3]);
     } else {
-      rank_skip = kEncBucketBackoff;
-      __syncwarp();  // S is read back before the warp sort writes it
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        *reinterpret_cast<uint2 *>(sm.R + 256 * h + 2 * t) = make_uint2(rel[2 * h], rel[2 * h + 1]);
     }
+    orv = __reduce_or_sync(FULL, orv);
+    if (lane == 0) sm.relor[warp] = orv;
+  }
+  if (pending && sm.goff != kGoffPending) {
+    place_parked<T>(pa[pk.head], sm, pk.head);
+    pk.head = pk.head + 1u < (uint32_t)kEncSlots ? pk.head + 1u : 0u;
+    --pk.count;
+    pending = false;
+  }
+
+  // ---- 2. rank the composites (block id, r) ----
+  const bool narrow = bound < (1u << 22);
+  int how = 0;  // 0: radix, 1: narrow buckets, 2: wide buckets
+  if (full && bound >= (1u << kEncBucketBits) && rank_skip == 0u) {
+    if (narrow) how = rank_buckets<T, true>(sm, H, S, key, bound, t, lane, warp) ? 1 : 0;
+    else how = rank_buckets<T, false>(sm, H, S, key, bound, t, lane, warp) ? 2 : 0;
+    // one crowded bucket says little about the next chunk (a shuffled, clustered
+    // snapshot has a few); a second one in a row does (ordered points)
+    if (how != 0) declined = 0u;
+    else if (++declined >= 2u) rank_skip = kEncBucketBackoff;
   } else if (rank_skip != 0u) {
     --rank_skip;
   }
-  if (!ranked) {
-    // 32-bit composites: one data-independent warp sort.  Slots past the
-    // chunk's end (point 32j + lane >= nvalid) take the largest
-    // composite, (kmax - kmin) << 10 | 1023: no point of a short chunk has
-    // r = 1023, so they sort last, and they carry the last id kmax, so they
-    // start no run.
+  const uint16_t *ranks = reinterpret_cast<const uint16_t *>(sm.Q);
+  if (how == 0) {
+    const uint32_t rbase = Points<T>::rank_base(t);
+    if (!full) {  // slots past the end sort last
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      key[j] = (full || 32u * j + lane < nvalid) ? (((key[j] - kmin) << 10) | (32u * lane + j)) : (uint32_t)cmax;
-#pragma unroll
-    for (int m = 0; m < 8; ++m)
-      *reinterpret_cast<uint4 *>(S + qoff(lane, m)) = make_uint4(key[4 * m], key[4 * m + 1], key[4 * m + 2], key[4 * m + 3]);
-    warp_sort1024_rows(S, hist, lane);
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const uint4 t = *reinterpret_cast<const uint4 *>(S + qoff(lane, m));
-      key[4 * m] = t.x; key[4 * m + 1] = t.y; key[4 * m + 2] = t.z; key[4 * m + 3] = t.w;
+      for (int e = 0; e < kEncPer; ++e)
+        if (Points<T>::point(t, e) >= nvalid) key[e] = bound + 1u;
     }
 #pragma unroll
-    for (int k = 0; k < 16; ++k) rp[k] = (key[k] & 1023u) | ((key[k + 16] & 1023u) << 16);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) key[j] = kmin + (key[j] >> 10);
+    for (int e = 0; e < kEncPer; ++e) S[rx(rbase + Points<T>::rank_step(e))] = key[e];
+    ranks = radix_rank(S, H, reinterpret_cast<uint16_t *>(sm.Q), sm.tot, bitlen(bound + (full ? 0u : 1u)));
   }
-  __syncwarp();  // ranking scratch is done with
 
   // ---- 3. runs: unique ids, deltas, counts (:222-311) ----
-  uint32_t *const runStart = sw, *const deltaA = sw + kChunk;
-  uint32_t U, dbits, cbits, first;
+  // thread t takes positions 128j + t, so that neighbouring lanes hold
+  // neighbouring positions and write neighbouring runs
+  if (warp == 2) claim();
+  uint32_t U, dbits, cbits;
   {
-    // ids ascend, so a run starts where the id differs from its predecessor,
-    // and the widest delta is the bit length of all deltas ORed together;
-    // position 0 starts the first run with delta 0.  Positions past the end
-    // repeat kmax and start no run.
-    const uint32_t prevk = __shfl_up_sync(FULL, key[31], 1);
-    const uint32_t pk0 = lane == 0 ? key[0] : prevk;
-    uint32_t fm = lane == 0 ? 1u : 0u, dm = 0;
-    if constexpr (!is64) {
-      uint32_t dor = 0;
+    uint32_t id[8], rel[8], starts[8];  // id: then the delta; starts: the warp's run starts
+    if (how == 1) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const uint32_t dlt = key[j] - (j ? key[j - 1] : pk0);
-        dor |= dlt;
-        if (dlt != 0u) fm |= 1u << j;
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t k = H[128 * j + t];
+        const uint32_t kp = (j == 0 && t == 0) ? k : H[128 * j + t - 1];
+        rel[j] = sm.R[point_of_rank(k & 1023u)];
+        if (j == 0 && t == 0) sm.first = k >> 10;
+        id[j] = (k >> 10) - (kp >> 10);
       }
-      dm = bitlen(dor);
-    } else {  // the same result; this form keeps the double kernels' registers lower
+    } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const uint32_t dlt = key[j] - (j ? key[j - 1] : pk0);
-        if (dlt != 0u) {
-          fm |= 1u << j;
-          dm = max(dm, bitlen(dlt));
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t p = 128u * j + t, pp = p == 0u ? 0u : p - 1u;
+        const uint32_t r = (uint32_t)ranks[p], k = how == 2 ? H[p] : S[rx(r)];
+        const uint32_t kp = how == 2 ? H[pp] : S[rx((uint32_t)ranks[pp])];
+        rel[j] = sm.R[point_of_rank(r)];
+        if (p == 0u) sm.first = k;
+        id[j] = k - kp;
+        if (p >= nvalid) {  // past the end: no run; relative positions all ones (:197)
+          id[j] = 0u;
+          rel[j] = FULL;
         }
       }
     }
-    const uint32_t cnt = __popc(fm);
-    uint32_t inc = cnt;
+    uint32_t dor = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(FULL, inc, o);
-      if (lane >= o) inc += t;
+    for (int j = 0; j < 8; ++j) {
+      dor |= id[j];
+      starts[j] = __ballot_sync(FULL, id[j] != 0u || (j == 0 && t == 0));
     }
+    dor = __reduce_or_sync(FULL, dor);
+    if (lane == 0) {
+      *reinterpret_cast<uint4 *>(sm.seg + 8 * warp) =
+          make_uint4(__popc(starts[0]), __popc(starts[1]), __popc(starts[2]), __popc(starts[3]));
+      *reinterpret_cast<uint4 *>(sm.seg + 8 * warp + 4) =
+          make_uint4(__popc(starts[4]), __popc(starts[5]), __popc(starts[6]), __popc(starts[7]));
+      sm.dor[warp] = dor;
+    }
+    __syncthreads();  // run counts; the ranking's arrays have been read
+    if (pending && warp == 3) look_up<T>(pa[pk.head], pk.head, sm, true, lane);
+    // lane i: the runs that start in positions 32i..32i+31 (row i = 4j + warp)
+    const uint32_t row = sm.seg[8 * (lane & 3) + (lane >> 2)];
+    const uint32_t inc = warp_inc_scan(row, lane), exc = inc - row;
     U = __shfl_sync(FULL, inc, 31);
-    dbits = warp_max(dm);
-    first = __shfl_sync(FULL, key[0], 0);
-    uint32_t u = inc - cnt;
+    const uint4 d4 = ld4(sm.dor);
+    dbits = bitlen(d4.x | d4.y | d4.z | d4.w);
+    const uint32_t below = (1u << lane) - 1u;
+    // swizzled index of position 128j + t: rows 4j + warp, quads XORed by the row
+    const uint32_t x0 = 32u * warp + (lane ^ (4u * warp));
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      if ((fm >> j) & 1u) {
-        runStart[sx(u)] = 32u * lane + j;
-        deltaA[sx(u)] = key[j] - (j ? key[j - 1] : pk0);
-        ++u;
+    for (int j = 0; j < 8; ++j) {
+      sm.Q[128 * j + (j & 1 ? x0 ^ 16u : x0)] = rel[j];
+      const uint32_t u = __shfl_sync(FULL, exc, 4 * j + warp) + __popc(starts[j] & below);
+      if ((starts[j] >> lane) & 1u) {
+        const uint32_t i = sx(u);
+        S[i] = 128u * j + t;
+        H[i] = id[j];
       }
     }
+    // the last, partly filled row of deltas ends in zeros
+    if (warp == 1 && U + lane < (uint32_t)kChunk) H[sx(U + lane)] = 0u;
   }
-  __syncwarp();
-  // this lane's runs 32l..32l+31: deltas, and counts as 16-bit pairs
-  uint32_t dl[32], cp[16];
+  __syncthreads();  // run starts and deltas, the parked chunk's offset
+  if (pending) {
+    place_parked<T>(pa[pk.head], sm, pk.head);
+    pk.head = pk.head + 1u < (uint32_t)kEncSlots ? pk.head + 1u : 0u;
+    --pk.count;
+  }
+  // thread t takes runs 8t..8t+7
   {
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const uint4 t = *reinterpret_cast<const uint4 *>(runStart + qoff(lane, m));
-      const uint4 q = *reinterpret_cast<const uint4 *>(deltaA + qoff(lane, m));
-      key[4 * m] = t.x; key[4 * m + 1] = t.y; key[4 * m + 2] = t.z; key[4 * m + 3] = t.w;
-      dl[4 * m] = q.x; dl[4 * m + 1] = q.y; dl[4 * m + 2] = q.z; dl[4 * m + 3] = q.w;
+    const uint32_t q0 = qoff(t >> 2, (2 * t) & 7), q1 = qoff(t >> 2, (2 * t + 1) & 7);
+    uint32_t st[9];
+    {
+      const uint4 u0 = ld4(S + q0), u1 = ld4(S + q1);
+      st[0] = u0.x; st[1] = u0.y; st[2] = u0.z; st[3] = u0.w;
+      st[4] = u1.x; st[5] = u1.y; st[6] = u1.z; st[7] = u1.w;
     }
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const bool live = 32u * lane + j < U;
-      key[j] = live ? key[j] : nvalid;
-      dl[j] = live ? dl[j] : 0u;
-    }
-    const uint32_t nx = __shfl_down_sync(FULL, key[0], 1);
+    for (int j = 0; j < 8; ++j) st[j] = 8u * t + j < U ? st[j] : nvalid;
+    st[8] = __shfl_down_sync(FULL, st[0], 1);
+    if (lane == 31) st[8] = 8u * t + 8u < U ? S[sx(8u * t + 8u)] : nvalid;
     uint32_t cm = 0;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const uint32_t e = j < 31 ? key[j + 1] : (lane < 31 ? nx : nvalid);
-      key[j] = e - key[j];  // run length (0 past the last run)
-      cm = max(cm, key[j]);
+    for (int j = 0; j < 8; ++j) {
+      st[j] = st[j + 1] - st[j];  // run length (0 past the last run)
+      cm = max(cm, st[j]);
     }
-#pragma unroll
-    for (int k = 0; k < 16; ++k) cp[k] = key[k] | (key[k + 16] << 16);
-    cbits = bitlen(warp_max(cm));
+    *reinterpret_cast<uint4 *>(sm.R + q0) = make_uint4(st[0], st[1], st[2], st[3]);
+    *reinterpret_cast<uint4 *>(sm.R + q1) = make_uint4(st[4], st[5], st[6], st[7]);
+    cm = warp_max(cm);
+    if (lane == 0) sm.cmax[warp] = cm;
   }
-  __syncwarp();  // run rows read: the region becomes the payload staging
+  if (warp == 2) commit();
+  __syncthreads();  // run lengths, the next chunk; the parked payload is placed
+  cbits = bitlen(max4(ld4(sm.cmax)));
+  const uint4 r4 = ld4(sm.relor);
+  const uint32_t rbits = max(bitlen(r4.x | r4.y | r4.z | r4.w), full ? 0u : 1u);  // :200-201
 
   // ---- 4. bit planes -> staged payload (:313-411) ----
   const uint32_t db = section_bytes(U, dbits, Tr::pad), cb = section_bytes(U, cbits, Tr::pad);
   const uint32_t rb = rel_section_bytes(rbits, Tr::pad);
-  on_size(db + cb + rb);  // the payload size is known before its planes are built
+  if (t == 0) {
+    sm.park[(pk.head + pk.count) % (uint32_t)kEncSlots] = {c, db + cb + rb};
+    publish_size(a.ctl, a.look, c, db + cb + rb);
+    uint32_t *m = reinterpret_cast<uint32_t *>(a.out + Tr::hdr + 8ull * a.G + (unsigned long long)Tr::meta * c);
+    if constexpr (!is64) {
+      m[6] = sm.first;
+      m[7] = dbits | (cbits << 16);
+      m[8] = rbits | (U << 16);
+    } else {
+      m[12] = sm.first;
+      m[13] = 0u;
+      m[14] = dbits | (cbits << 16);
+      m[15] = rbits | (U << 16);
+    }
+  }
+  const uint32_t slot = (pk.head + pk.count) % (uint32_t)kEncSlots;
+  ++pk.count;
   const uint32_t bpp = (U + 7u) >> 3;
-  uint32_t *const stage = sw;
-  put_planes(stage, 0u, dbits, bpp, dl, lane);
-#pragma unroll
-  for (int k = 0; k < 16; ++k) { dl[k] = cp[k] & 0xFFFFu; dl[k + 16] = cp[k] >> 16; }
-  put_planes(stage, db, cbits, bpp, dl, lane);
-  // delta + count sections end below 8 KB: the rank rows are still intact
-#pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    const uint32_t r = (rp[j & 15] >> (16 * (j >> 4))) & 1023u;
-    dl[j] = relR[sx(r)];
-  }
-  if (!full) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (32u * lane + j >= nvalid) dl[j] = 0xFFFFFFFFu;  // slots past the end (:197)
-  }
-  __syncwarp();
-  put_planes(stage, db + cb, rbits, 0u, dl, lane);
+  uint8_t *const stage = reinterpret_cast<uint8_t *>(sm.P[slot]);
   {
+    // jobs of eight planes, the longest first
+    const uint32_t nd = (dbits + 7u) >> 3, nr = (rbits + 7u) >> 3, nc = (cbits + 7u) >> 3;
+    for (uint32_t j = warp; j < nd + nr + nc; j += kEncWarps) {
+      if (j - nd < nr) plane_job<8>(sm.Q, stage, db + cb, rbits, 8u * (j - nd), 0u, lane);
+      else if (j < nd) plane_job<8>(H, stage, 0u, dbits, 8u * j, bpp, lane);
+      else plane_job<8>(sm.R, stage, db, cbits, 8u * (j - nd - nr), bpp, lane);
+    }
+  }
+  if (warp == kEncWarps - 1) {
     // section padding is zero (the reference leaves it unwritten)
-    uint8_t *stage8 = reinterpret_cast<uint8_t *>(stage);
-    const uint32_t p0 = dbits * bpp + lane, p1 = db + cbits * bpp + lane;
-    if (p0 < db) stage8[p0] = 0;
-    if (p1 < db + cb) stage8[p1] = 0;
+    const uint32_t a0 = dbits * bpp + lane, a1 = db + cbits * bpp + lane;
+    if (a0 < db) stage[a0] = 0;
+    if (a1 < db + cb) stage[a1] = 0;
   }
-
-  // meta record (:332-344 / Double :333-345)
-  {
-    uint32_t w = 0;
-    if (!is64) {
-      if (lane < 6) w = mword;
-      if (lane == 6) w = first;
-      if (lane == 7) w = dbits | (cbits << 16);
-      if (lane == 8) w = rbits | (U << 16);
-    } else {
-      if (lane < 12) w = mword;
-      if (lane == 12) w = first;
-      if (lane == 13) w = 0;
-      if (lane == 14) w = dbits | (cbits << 16);
-      if (lane == 15) w = rbits | (U << 16);
-    }
-    meta_word = w;
-  }
-  return db + cb + rb;
+  return slot;
 }
 
-// Encodes chunk c into the warp's region `sw`; returns the payload bytes and
-// leaves the meta record in meta_word (word k of the record in lane k).
-// on_size(bytes) runs (warp-wide) as soon as the payload size is known, before
-// the bit planes are built.  rank_skip is the warp's count of chunks still to
-// rank by the warp sort without trying the buckets first.
-template <typename T, int DIM, class OnSize>
-__device__ __forceinline__ uint32_t encode_chunk(const CArgs<T> &a, unsigned long long c, uint32_t *sw,
-                                                 uint32_t seg, uint32_t sh, uint32_t msk, T eb, T inv,
-                                                 ChunkPoints<T, DIM> &pts, uint32_t &meta_word, int lane,
-                                                 uint32_t &rank_skip, OnSize &&on_size) {
-  ChunkQ q;
-  encode_quantize<T, DIM>(a, c, sw, seg, sh, msk, eb, inv, pts, q, lane);
-  return encode_pack<T, DIM>(a, c, sw, q, meta_word, lane, rank_skip, on_size);
-}
-
-// Copies a staged payload (whole words) to its place in the stream: four
-// independent shared loads per lane before their global stores, so the loads'
-// latency is paid once per 512 bytes rather than per 128.
-__device__ __forceinline__ void copy_payload(uint32_t *dst, const uint32_t *sw, uint32_t payload, int lane) {
-  const uint32_t nw = payload / 4u;
-  for (uint32_t w = lane; w < nw; w += 128) {
-    uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0;
-    if (w < nw) t0 = sw[w];
-    if (w + 32 < nw) t1 = sw[w + 32];
-    if (w + 64 < nw) t2 = sw[w + 64];
-    if (w + 96 < nw) t3 = sw[w + 96];
-    if (w < nw) dst[w] = t0;
-    if (w + 32 < nw) dst[w + 32] = t1;
-    if (w + 64 < nw) dst[w + 64] = t2;
-    if (w + 96 < nw) dst[w + 96] = t3;
+// Places what is parked when the work has run out.
+template <typename T, class PArgs>
+__device__ __forceinline__ void flush_parked(const PArgs &pa, EncShared &sm, Parked &pk, int lane, int warp) {
+  for (; pk.count != 0u; --pk.count) {
+    __syncthreads();
+    if (warp == 0) look_up<T>(pa[pk.head], pk.head, sm, true, lane);
+    __syncthreads();
+    place_parked<T>(pa[pk.head], sm, pk.head);
+    pk.head = pk.head + 1u < (uint32_t)kEncSlots ? pk.head + 1u : 0u;
   }
 }
 
-// Writes a placed chunk: its offset-table entry (:1679), meta record, payload,
-// and for chunk 0 the header (:1674-1678; Double :1672-1680).
+// The arguments of a parked chunk, when all chunks share them.
 template <typename T>
-__device__ __forceinline__ void place_chunk(const CArgs<T> &a, unsigned long long c, unsigned long long G,
-                                            unsigned long long pay_base, unsigned long long off, uint32_t payload,
-                                            uint32_t meta_word, uint32_t seg, T eb, const uint32_t *sw, int lane) {
-  using Tr = TT<T>;
-  constexpr bool is64 = sizeof(T) == 8;
-  if (lane == 0) reinterpret_cast<unsigned long long *>(a.out + Tr::hdr)[c] = off;
-  uint8_t *meta = a.out + Tr::hdr + 8ull * G + (unsigned long long)Tr::meta * c;
-  if (lane < (int)(Tr::meta / 4)) reinterpret_cast<uint32_t *>(meta)[lane] = meta_word;
-  if (c == 0) {
-    uint32_t *h = reinterpret_cast<uint32_t *>(a.out);
-    if (lane == 0) h[0] = a.dim;
-    if (lane == 1) h[1] = (uint32_t)a.n;
-    if (lane == 2) h[2] = (uint32_t)(a.n >> 32);
-    if (lane == 3) h[3] = Tr::bits;
-    if (!is64) {
-      if (lane == 4) h[4] = __float_as_uint((float)eb);
-      if (lane == 5) h[5] = seg;
-    } else {
-      if (lane == 4) h[4] = (uint32_t)__double_as_longlong((double)eb);
-      if (lane == 5) h[5] = (uint32_t)((unsigned long long)__double_as_longlong((double)eb) >> 32);
-      if (lane == 6) h[6] = seg;
-      if (lane == 7) h[7] = 32u;
-    }
-  }
-  if (pay_base + off + payload > a.out_cap) {
-    if (lane == 0) set_status(a.ctl, kENOSPACE);
-  } else {
-    copy_payload(reinterpret_cast<uint32_t *>(a.out + pay_base + off), sw, payload, lane);
-  }
-  if (c == G - 1 && lane == 0) a.ctl->stream_bytes = pay_base + off + payload;
-}
+struct SameArgs {
+  const CArgs<T> &a;
+  __device__ __forceinline__ const CArgs<T> &operator[](uint32_t) const { return a; }
+};
 
-// Persistent compress kernel: every CTA encodes groups of W consecutive
-// chunks, one chunk per warp.  Per group: the warps quantize,
-// rank and find the runs of their chunks; their payload sizes are then known
-// (barrier B1) and warp 0 publishes the group's aggregate, so that later
-// groups' look-backs can pass it while the warps build their bit planes;
-// warp 0 then resolves the group's stream offset (decoupled look-back) and
-// after barrier B2 every warp copies its staged payload out.
-template <typename T, int DIM, int W = enc_warps<T, DIM>()>
-__global__ void __launch_bounds__(32 * W, GPZ_ENC_MIN_CTAS) compress_kernel(const CArgs<T> a) {
-  using Tr = TT<T>;
+// Persistent compress kernel: every CTA claims one chunk after another.  A
+// chunk's payload size is published as soon as its runs are known and its
+// payload stays parked in shared memory; the CTA looks up its stream offset
+// (decoupled look-back) an iteration later without waiting, and waits for a
+// predecessor only when the room is needed for the next payload.
+template <typename T, int DIM>
+__global__ void __launch_bounds__(kEncThreads, kEncCtas) compress_kernel(const __grid_constant__ CArgs<T> a) {
   constexpr bool is64 = sizeof(T) == 8;
-  constexpr uint32_t FULL = 0xFFFFFFFFu;
-  extern __shared__ __align__(16) uint32_t enc_smem[];
-  __shared__ EncGroupT<W> eg;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t *const sw = enc_smem + warp * kEncWords;
+  extern __shared__ __align__(16) unsigned char enc_smem[];
+  EncShared &sm = *reinterpret_cast<EncShared *>(enc_smem);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   Control *ctl = a.ctl;
-  if (ld_volatile(reinterpret_cast<const uint32_t *>(&ctl->status)) != 0) return;
   const uint32_t seg = ctl->seg;
-  const uint32_t sh = (uint32_t)__ffs((int)seg) - 1u, msk = seg - 1u;
   const T eb = a.eb_dev ? (T)*a.eb_dev : a.eb;
   const T inv = is64 ? (T)__ddiv_rn(1.0, __dmul_rn(2.0, (double)eb)) : (T)__fdiv_rn(1.0f, __fmul_rn(2.0f, (float)eb));
   const unsigned long long G = a.G;
-  const unsigned long long pay_base = Tr::hdr + 8ull * G + (unsigned long long)Tr::meta * G;
-
-  if (threadIdx.x == 0) eg.next = atomicAdd(&ctl->chunk_ctr, (uint32_t)W);
-  __syncthreads();
-  ChunkPoints<T, DIM> pts;
-  pts.load(a, eg.next + warp, lane);
-  uint32_t rank_skip = 0;
-  for (;;) {
-    const unsigned long long gbase = eg.next;
-    if (gbase >= G) break;
-    __syncthreads();  // B0: everyone has the group before it is replaced
-    if (threadIdx.x == 0) eg.next = ld_volatile(&ctl->abort) ? G : atomicAdd(&ctl->chunk_ctr, (uint32_t)W);
-    const unsigned long long c = gbase + warp;
-    const unsigned long long gid = gbase / W;
-    uint32_t total = 0;
-    auto on_size = [&](uint32_t bytes) {
-      if (lane == 0) eg.sz[warp] = bytes;
-      __syncthreads();  // B1: the group's sizes are known
-      if (warp == 0) {
-        const uint32_t s = lane < W ? eg.sz[lane] : 0u;
-        total = __reduce_add_sync(FULL, s);
-        if (lane == 0) publish_aggregate(a.look, gid, total);
-      }
-    };
-    uint32_t payload = 0, meta_word = 0;
-    if (c < G) payload = encode_chunk<T, DIM>(a, c, sw, seg, sh, msk, eb, inv, pts, meta_word, lane, rank_skip, on_size);
-    else on_size(0u);
-    if (warp == 0) {
-      // resolved only now: the predecessors have had this group's plane
-      // building to publish, so the look-back rarely waits
-      unsigned long long excl = 0;
-      const bool ok = resolve_prefix(a.look, gid, total, ctl, excl);
-      if (lane == 0) eg.goff = ok ? excl : ~0ull;
-    }
-    pts.load(a, eg.next + warp, lane);  // in flight during the copy-out
-    __syncthreads();  // B2: the group's stream offset is known
-    const unsigned long long goff = eg.goff;
-    if (c < G && goff != ~0ull) {
-      unsigned long long off = goff;
-      for (int w = 0; w < warp; ++w) off += eg.sz[w];
-      place_chunk<T>(a, c, G, pay_base, off, payload, meta_word, seg, eb, sw, lane);
-    }
+  // nothing is claimed after a failure (sampling, bound, another CTA's)
+  if (t == 0) {
+    sm.overflowed = nullptr;
+    sm.next[0] = ld_volatile(reinterpret_cast<const uint32_t *>(&ctl->status)) != 0u
+                     ? G
+                     : (unsigned long long)atomicAdd(&ctl->chunk_ctr, 1u);
   }
+  __syncthreads();
+  Parked pk = {0u, 0u};
+  uint32_t rank_skip = 0, declined = 0, claimed = 0;
+  int par = 0;
+  for (;;) {
+    const unsigned long long c = sm.next[par];
+    if (c >= G) break;
+    encode_chunk<T, DIM>(
+        a, c, sm, par, seg, eb, inv, SameArgs<T>{a}, pk, rank_skip, declined,
+        [&]() {
+          if (lane == 0) claimed = ld_volatile(&ctl->abort) ? 0xFFFFFFFFu : atomicAdd(&ctl->chunk_ctr, 1u);
+        },
+        [&]() {
+          claimed = __shfl_sync(0xFFFFFFFFu, claimed, 0);
+          if (lane == 0) sm.next[par ^ 1] = claimed;
+          prefetch_points<T, DIM>(a, claimed, lane);
+        });
+    par ^= 1;
+  }
+  flush_parked<T>(SameArgs<T>{a}, sm, pk, lane, warp);
   rewind_work_counter(ctl);
 }
 

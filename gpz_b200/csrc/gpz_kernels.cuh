@@ -344,7 +344,8 @@ template <typename T>
 __device__ __forceinline__ void seg_sample_block(const T *__restrict__ x, const T *__restrict__ y,
                                                  const T *__restrict__ z, uint64_t n, uint32_t dim, uint32_t seg_in,
                                                  int rel_mode, T rel_eb, T eb, int safe31, Control *ctl,
-                                                 unsigned block, unsigned nblocks, const double *eb_dev = nullptr) {
+                                                 unsigned block, unsigned nblocks, const double *eb_dev = nullptr,
+                                                 uint32_t *seg_out = nullptr) {
   using U = typename TT<T>::U;
   __shared__ U red[6][8];
   __shared__ int last;
@@ -402,6 +403,7 @@ __device__ __forceinline__ void seg_sample_block(const T *__restrict__ x, const 
     }
     const T ebv = eb_dev ? (T)*(const volatile double *)eb_dev : eb;
     const SegDecision sd = decide_seg<T>(mm, dim, seg_in, rel_mode, rel_eb, ebv, safe31);
+    if (seg_out) *seg_out = sd.status == kOK ? sd.seg : 0u;
     if (sd.status != kOK) set_status(ctl, sd.status);
     else {
       ctl->seg = sd.seg;
@@ -544,68 +546,121 @@ struct CArgs {
   uint8_t *out;
   unsigned long long out_cap;
   Control *ctl;
-  unsigned long long *look;  // one look-back word per chunk
+  unsigned long long *look;  // look-back records (16-byte aligned)
   unsigned long long n, G;
   T eb;
   const double *eb_dev;  // when set, the bound is read here on the device (strict-bound mode)
   uint32_t dim;
-  int vec_ok;  // x, y, z all 16-byte aligned
 };
 
-constexpr unsigned long long kFlagAgg = 1ull << 62, kFlagInc = 2ull << 62, kValMask = (1ull << 62) - 1;
+// ---------------------------------------------------------------------------
+// Decoupled look-back over the chunk sizes.  One 32-byte record (four 64-bit
+// words) serves 16 chunks: their payload sizes in 4-byte units, 12 bits each
+// (five to a word, the sixteenth on top of the last word; zero until it is
+// known), and below that the group's prefix -- the stream offset of its first
+// chunk in 4-byte units -- with kLookKnown once somebody has it.  Every field
+// is set by one relaxed atomic OR and valid by itself, so neither side needs
+// a fence (an offset kept beside its flag cost two per chunk, 4-5 thousand
+// cycles under load).
+//
+// A chunk's offset is the nearest known prefix at or below its own group plus
+// the sizes from there on; a step reads 512 predecessors, one record a lane,
+// since with over a thousand chunks in flight the nearest prefix is a few
+// hundred chunks back.  Record 0 stands in the control block's last 32 bytes,
+// the others follow at `look` + 4 words a record.
+// ---------------------------------------------------------------------------
+constexpr int kLookGroup = 16;
+constexpr unsigned long long kLookKnown = 1ull << 51, kLookPrefix = kLookKnown - 1;
+constexpr int kLookTail = kCtlBytes - 32;  // record 0 in the control block
+static_assert(sizeof(Control) <= kLookTail, "record 0 must not touch the control fields");
+static_assert(kStageBytes / 4 < 4096, "payload size in 12 bits");
 
-// Decoupled look-back over the chunk sizes.  A chunk publishes its own
-// payload size (aggregate) as soon as it knows it; placing it later
-// (resolve_prefix, one CTA iteration afterwards) sums the aggregates of its
-// predecessors back to the nearest published inclusive prefix, then
-// publishes its own inclusive prefix.
-__device__ __forceinline__ void publish_aggregate(unsigned long long *look, unsigned long long c,
-                                                  unsigned long long agg) {
-  st_relaxed(&look[c], (c == 0 ? kFlagInc : kFlagAgg) | agg);
+// Bytes of the records after the first, for G chunks.
+__host__ __device__ inline unsigned long long look_bytes(unsigned long long G) {
+  return 32ull * ((G + kLookGroup - 1) / kLookGroup - 1);
 }
 
-// Warp-collective.  Returns false when a bounded wait (`limit` polls of a
-// predecessor that has published nothing) gave up or another CTA aborted (the
-// kernel then stops taking chunks and reports GPZ_ETIMEOUT).
-static __device__ bool resolve_prefix(unsigned long long *look, unsigned long long c, unsigned long long agg,
-                                      Control *ctl, unsigned long long &excl_out, uint32_t limit = kSpinLimit) {
+__device__ __forceinline__ unsigned long long *look_record(Control *ctl, unsigned long long *look,
+                                                           unsigned long long g) {
+  return g == 0 ? reinterpret_cast<unsigned long long *>(reinterpret_cast<uint8_t *>(ctl) + kLookTail) : look + 4 * g;
+}
+
+// One thread: the payload size of chunk c (bytes, a multiple of 4, not 0).
+__device__ __forceinline__ void publish_size(Control *ctl, unsigned long long *look, unsigned long long c,
+                                             uint32_t bytes) {
+  const uint32_t i = (uint32_t)c & (kLookGroup - 1u), w = i / 5u;  // chunk 15: word 3
+  const uint32_t sh = i == 15u ? 52u : 12u * (i - 5u * w);
+  red_or_relaxed(look_record(ctl, look, c / kLookGroup) + w, (unsigned long long)(bytes >> 2) << sh);
+}
+
+// Warp-collective: the stream offset of chunk c, and its group's prefix for
+// those behind.  Returns 1; while a predecessor has published nothing: -1
+// without `wait`; with it, polls up to `limit` times and returns 0 when that
+// or another CTA gave up (the kernel then stops taking chunks and reports
+// GPZ_ETIMEOUT).
+static __device__ int resolve_prefix(Control *ctl, unsigned long long *look, unsigned long long c,
+                                     unsigned long long &excl_out, uint32_t limit = kSpinLimit, bool wait = true) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
-  if (c == 0) {
-    excl_out = 0;
-    return true;
-  }
-  unsigned long long excl = 0;
-  long long top = (long long)c - 1;
+  const uint32_t own = (uint32_t)c & (kLookGroup - 1u);  // predecessors in the chunk's own group
+  long long top = (long long)(c / kLookGroup);           // group of lane 31
+  uint32_t in_group = 0;                                 // their sizes
+  unsigned long long excl = 0;                           // units
   uint32_t spins = 0, backoff = 32;
-  while (true) {
-    const long long idx = top - lane;
-    const unsigned long long v = idx >= 0 ? ld_relaxed(&look[idx]) : kFlagInc;
-    const uint32_t fl = (uint32_t)(v >> 62);
-    const uint32_t mInc = __ballot_sync(0xFFFFFFFFu, fl == 2u);
-    const uint32_t mNone = __ballot_sync(0xFFFFFFFFu, fl == 0u);
-    const uint32_t need = mInc ? (((mInc & (0u - mInc)) << 1) - 1u) : 0xFFFFFFFFu;
-    if (mNone & need) {
+  for (;;) {
+    const long long g = top - 31 + lane;
+    uint4 q0 = make_uint4(0u, 0u, 0u, 0u), q1 = q0;
+    if (g >= 0) {
+      const uint4 *const rec = reinterpret_cast<const uint4 *>(look_record(ctl, look, (unsigned long long)g));
+      q0 = ld_relaxed4(rec);
+      q1 = ld_relaxed4(rec + 1);
+    }
+    const unsigned long long w3 = ((unsigned long long)q1.w << 32) | q1.z;
+    const bool known = g <= 0 || (w3 & kLookKnown) != 0ull;
+    const int near = 31 - __clz((int)__ballot_sync(FULL, known));  // -1: none in the window
+    // sizes of this lane's chunks before c
+    const uint32_t cnt = g == (long long)(c / kLookGroup) ? own : (uint32_t)kLookGroup;
+    const uint32_t lo[3] = {q0.x, q0.z, q1.x}, hi[3] = {q0.y, q0.w, q1.y};
+    uint32_t sum = 0;
+    bool missing = false;
+#pragma unroll
+    for (uint32_t i = 0; i < (uint32_t)kLookGroup; ++i) {
+      const uint32_t w = i < 15u ? i / 5u : 2u, sh = 12u * (i % 5u);
+      const uint32_t v = i == 15u ? q1.w >> 20
+                                  : (sh >= 32u ? hi[w] >> (sh - 32u) : __funnelshift_r(lo[w], hi[w], sh)) & 4095u;
+      if (i < cnt) {
+        sum += v;
+        missing |= v == 0u;
+      }
+    }
+    const bool counts = g >= 0 && lane >= near;
+    if (__any_sync(FULL, counts && missing)) {
+      if (!wait) return -1;
       if (++spins > limit || ld_volatile(&ctl->abort)) {
         if (lane == 0) {
           atomicExch(&ctl->abort, 1u);
           set_status(ctl, kETIMEOUT);
         }
-        return false;
+        return 0;
       }
       __nanosleep(backoff);
       backoff = min(backoff * 2, 256u);
       continue;
     }
-    unsigned long long add = ((need >> lane) & 1u) ? (v & kValMask) : 0ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xFFFFFFFFu, add, o);
-    excl += add;
-    if (mInc) break;
+    excl += __reduce_add_sync(FULL, counts ? sum : 0u);
+    if (top == (long long)(c / kLookGroup)) in_group = __shfl_sync(FULL, sum, 31);
+    if (near >= 0) {
+      const unsigned long long pre = g <= 0 ? 0ull : (w3 & kLookPrefix);
+      excl += __shfl_sync(FULL, pre, near);
+      // the group's prefix, unless it is there (setting it again changes nothing)
+      if (lane == 31 && !(top == (long long)(c / kLookGroup) && near == 31))
+        red_or_relaxed(look_record(ctl, look, c / kLookGroup) + 3, kLookKnown | (excl - in_group));
+      break;
+    }
     top -= 32;
   }
-  if (lane == 0) st_relaxed(&look[c], kFlagInc | (excl + agg));
-  excl_out = excl;
-  return true;
+  excl_out = 4ull * excl;
+  return 1;
 }
 
 }  // namespace gpzb
