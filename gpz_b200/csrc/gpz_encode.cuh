@@ -92,29 +92,33 @@ __device__ __forceinline__ double max2(double a, double b) { return from_ord(max
 // row apart) and read in any order: the row's five bits XORed into the bank.
 __device__ __forceinline__ uint32_t rx(uint32_t r) { return r ^ (r >> 5); }
 
-// A CTA's shared memory.
-struct EncShared {
-  uint32_t A[2][kChunk];         // bucket counts -> sorted composites -> deltas | placed composites -> run starts
-                                 // (roles alternate from chunk to chunk: clearing the counts needs no barrier)
+// Shared memory of the ranking of a chunk.
+struct RankShared {
+  __align__(16) uint32_t A[2][kChunk];  // bucket counts -> sorted composites -> deltas | placed composites -> run starts
+                                        // (roles alternate from chunk to chunk: clearing the counts needs no barrier)
   uint32_t R[kChunk];            // relative positions by point -> run lengths
   uint32_t Q[kChunk];            // ranks in sorted order (not of narrow chunks) -> relative positions in that order
-  uint32_t P[kEncSlots][kStageBytes / 4];  // staged payloads
-  struct { unsigned long long c; uint32_t payload; } park[kEncSlots];  // their chunks and sizes
-  unsigned long long goff;       // stream offset of the parked chunk (kGoffPending, kGoffNone: none)
-  unsigned long long next[2];    // chunk claimed for the next iteration, by parity
   __align__(16) double mm[kEncWarps][8];   // warps' minima (0..2) and maxima (4..6), in the stream's type
   __align__(16) double nm[4];    // chunk: -min / (2 eb) per axis, in the stream's type
   __align__(16) uint32_t sc[4];  // chunk: id multipliers of y and z, largest id
   __align__(16) uint32_t tot[kEncWarps];   // per-warp sums of the bucket / digit scans
   __align__(16) uint32_t big[kEncWarps];   // per-warp largest bucket
-  __align__(16) uint32_t relor[kEncWarps]; // OR of the relative positions
-  __align__(16) uint32_t seg[8 * kEncWarps];  // run starts per 32 positions: [warp][j]
-  __align__(16) uint32_t dor[kEncWarps];   // OR of the deltas
-  __align__(16) uint32_t cmax[kEncWarps];  // longest run
   __align__(16) uint32_t cpts[kEncWarps];  // points in buckets of kEncSmall or more
   __align__(16) uint32_t small[kEncWarps]; // per-warp largest bucket below that
   uint32_t crowd[kEncCrowdPoints / kEncSmall];  // those buckets: first position << 16 | points
   uint32_t ncrowd;
+};
+
+// A compress CTA's shared memory.
+struct EncShared : RankShared {
+  __align__(16) uint32_t P[kEncSlots][kStageBytes / 4];  // staged payloads
+  struct { unsigned long long c; uint32_t payload; } park[kEncSlots];  // their chunks and sizes
+  unsigned long long goff;       // stream offset of the parked chunk (kGoffPending, kGoffNone: none)
+  unsigned long long next[2];    // chunk claimed for the next iteration, by parity
+  __align__(16) uint32_t relor[kEncWarps]; // OR of the relative positions
+  __align__(16) uint32_t seg[8 * kEncWarps];  // run starts per 32 positions: [warp][j]
+  __align__(16) uint32_t dor[kEncWarps];   // OR of the deltas
+  __align__(16) uint32_t cmax[kEncWarps];  // longest run
   uint32_t first;                // smallest block id
   Control *overflowed;           // stream whose id_overflow this CTA has set last
 };
@@ -376,7 +380,7 @@ struct Points {
 // crowded buckets (ordered snapshots) are cheaper in the radix sort: hence the
 // second limit.
 template <typename T, bool kNarrow>
-__device__ __forceinline__ bool rank_buckets(EncShared &sm, uint32_t *H, uint32_t *S, const uint32_t (&key)[kEncPer],
+__device__ __forceinline__ bool rank_buckets(RankShared &sm, uint32_t *H, uint32_t *S, const uint32_t (&key)[kEncPer],
                                              uint32_t bound, int t, int lane, int warp) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t rbase = Points<T>::rank_base(t);
@@ -537,13 +541,14 @@ __device__ __forceinline__ bool rank_buckets(EncShared &sm, uint32_t *H, uint32_
 }
 
 template <typename T, int DIM>
-__device__ __forceinline__ void load_points(const CArgs<T> &a, unsigned long long base, uint32_t nvalid,
-                                            T (&v)[DIM][kEncPer]) {
+__device__ __forceinline__ void load_points(const T *x, const T *y, const T *z, unsigned long long base,
+                                            uint32_t nvalid, T (&v)[DIM][kEncPer]) {
   constexpr int V = Points<T>::kVec;
   const uint32_t t = threadIdx.x;
-  const T *const X[3] = {a.x + base, a.y + base, a.z + base};
-  uint32_t low = (uint32_t)(uintptr_t)a.x | (uint32_t)(uintptr_t)a.y;
-  if (DIM == 3) low |= (uint32_t)(uintptr_t)a.z;
+  const T *const X[3] = {x + base, y + base, z + base};
+  uint32_t low = (uint32_t)(uintptr_t)x;
+  if (DIM >= 2) low |= (uint32_t)(uintptr_t)y;
+  if (DIM == 3) low |= (uint32_t)(uintptr_t)z;
   if (nvalid == (uint32_t)kChunk && (low & 15u) == 0u) {
 #pragma unroll
     for (int d = 0; d < DIM; ++d)
@@ -569,6 +574,22 @@ __device__ __forceinline__ void load_points(const CArgs<T> &a, unsigned long lon
   }
 }
 
+// The warp's minima and maxima into sm.mm.
+template <typename T, int DIM>
+__device__ __forceinline__ void put_minmax(RankShared &sm, const T (&v)[DIM][kEncPer], int lane, int warp) {
+  T mn[3], mx[3];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) warp_minmax(v[d], mn[d], mx[d]);
+  if (lane == 0) {
+    T *const m = reinterpret_cast<T *>(sm.mm[warp]);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      m[d] = mn[d];
+      m[4 + d] = mx[d];
+    }
+  }
+}
+
 // Asks for chunk c's axes in L2 (bulk prefetches of the 16-byte aligned
 // spans, one lane per axis), ahead of its load.
 template <typename T, int DIM>
@@ -581,6 +602,43 @@ __device__ __forceinline__ void prefetch_points(const CArgs<T> &a, unsigned long
     if (bytes != 0u && (reinterpret_cast<uintptr_t>(p) & 15u) == 0u)
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
   }
+}
+
+// Ranks a chunk's points by (block id, r): narrow buckets (1: H holds the
+// sorted composites), wide buckets (2: H the sorted ids, `ranks` the ranks) or
+// the radix sort (0: S the ids by rank, rx, `ranks` the ranks).  No id is above
+// `bound`; positions past the end of a short chunk rank last.  rank_skip counts
+// the chunks still to sort without trying the buckets, declined the chunks the
+// buckets have declined in a row.
+template <typename T>
+__device__ __forceinline__ int rank_chunk(RankShared &sm, uint32_t *H, uint32_t *S, uint32_t (&key)[kEncPer],
+                                          uint32_t bound, uint32_t nvalid, uint32_t &rank_skip, uint32_t &declined,
+                                          int t, int lane, int warp, const uint16_t *&ranks) {
+  const bool full = nvalid == (uint32_t)kChunk, narrow = bound < (1u << 22);
+  int how = 0;
+  if (full && bound >= (1u << kEncBucketBits) && rank_skip == 0u) {
+    if (narrow) how = rank_buckets<T, true>(sm, H, S, key, bound, t, lane, warp) ? 1 : 0;
+    else how = rank_buckets<T, false>(sm, H, S, key, bound, t, lane, warp) ? 2 : 0;
+    // one crowded chunk says little about the next (a shuffled, clustered
+    // snapshot has a few); a second one in a row does (ordered points)
+    if (how != 0) declined = 0u;
+    else if (++declined >= 2u) rank_skip = kEncBucketBackoff;
+  } else if (rank_skip != 0u) {
+    --rank_skip;
+  }
+  ranks = reinterpret_cast<const uint16_t *>(sm.Q);
+  if (how == 0) {
+    const uint32_t rbase = Points<T>::rank_base(t);
+    if (!full) {  // slots past the end sort last
+#pragma unroll
+      for (int e = 0; e < kEncPer; ++e)
+        if (Points<T>::point(t, e) >= nvalid) key[e] = bound + 1u;
+    }
+#pragma unroll
+    for (int e = 0; e < kEncPer; ++e) S[rx(rbase + Points<T>::rank_step(e))] = key[e];
+    ranks = radix_rank(S, H, reinterpret_cast<uint16_t *>(sm.Q), sm.tot, bitlen(bound + (full ? 0u : 1u)));
+  }
+  return how;
 }
 
 // The parked payloads of a CTA: `count` of them, the oldest in slot `head`.
@@ -648,13 +706,14 @@ __device__ __forceinline__ void look_up(const CArgs<T> &a, uint32_t slot, EncSha
   if (lane == 0) sm.goff = ok > 0 ? excl : (ok < 0 ? kGoffPending : kGoffNone);
 }
 
-// The chunk's scalars, by the first warp: per-axis values in lanes 0..2 (lane
-// d: axis d).  Block counts, id multipliers, offsets -min / (2 eb), the
-// largest block id, the meta record's min / max (:332-344 / Double :333-345).
+// The chunk's scalars, by one warp: per-axis values in lanes 0..2 (lane d:
+// axis d).  Block counts, id multipliers, offsets -min / (2 eb) and the largest
+// block id into sm.sc and sm.nm; returns the minimum (lane d) and maximum (lane
+// 3 + d) of axis d, and the axis's share of the largest corner's id (term; it
+// may not fit 31 bits when wide is set).
 template <typename T, int DIM>
-__device__ __forceinline__ void chunk_scalars(const CArgs<T> &a, unsigned long long c, EncShared &sm, uint32_t seg,
-                                              uint32_t sh, T eb, T inv, int lane) {
-  using Tr = TT<T>;
+__device__ __forceinline__ T chunk_scalars(RankShared &sm, uint32_t seg, uint32_t sh, T eb, T inv, int lane,
+                                           unsigned long long &term, bool &wide) {
   constexpr bool is64 = sizeof(T) == 8;
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   T mmv;
@@ -688,20 +747,34 @@ __device__ __forceinline__ void chunk_scalars(const CArgs<T> &a, unsigned long l
     bny = __shfl_sync(FULL, (uint32_t)bn, 1);
   }
   const unsigned long long mult = lane == 0 ? 1ull : (lane == 1 ? bnx : bnx * bny);
-  const unsigned long long term = lane < DIM ? (qm >> sh) * mult : 0ull;
+  term = lane < DIM ? (qm >> sh) * mult : 0ull;
   // the chunk's largest quantized corner: every quantized value is at most its
   // axis's (the multiply-add and the truncation are monotone), so no id is
   // above the sum; ids are masked to 31 bits when it does not fit
   const float tf = lane < DIM ? __ull2float_rn(qm >> sh) * __ull2float_rn(mult) : 0.0f;
-  const bool wide = __any_sync(FULL, tf >= 7.0e8f);
+  wide = __any_sync(FULL, tf >= 7.0e8f);
   const uint32_t sum = __reduce_add_sync(FULL, (uint32_t)term);
   if (lane < 3) reinterpret_cast<T *>(sm.nm)[lane] = nm;
   if (lane == 0) *reinterpret_cast<uint4 *>(sm.sc) = make_uint4((uint32_t)bnx, (uint32_t)(bnx * bny), wide ? 0x7FFFFFFFu : sum, 0u);
+  return mmv;
+}
+
+// The first warp's part of encoding chunk c between the barriers: its scalars,
+// the id_overflow flag, the meta record's min / max (:332-344 / Double
+// :333-345), the stream's header.
+template <typename T, int DIM>
+__device__ __forceinline__ void encode_scalars(const CArgs<T> &a, unsigned long long c, EncShared &sm, uint32_t seg,
+                                               uint32_t sh, T eb, T inv, int lane) {
+  using Tr = TT<T>;
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  unsigned long long term;
+  bool wide;
+  const T mmv = chunk_scalars<T, DIM>(sm, seg, sh, eb, inv, lane, term, wide);
   if (wide) {
-    // id_overflow: the same corner in u64 arithmetic (terms below 7e8 cannot
-    // reach 2^31).  Set once per CTA and stream: the flag shares its cache line
-    // with the work counter, and a store per chunk took 50M double points from
-    // 1.1 to 2.3 ms.
+    // id_overflow: the largest corner in u64 arithmetic (terms below 7e8
+    // cannot reach 2^31).  Set once per CTA and stream: the flag shares its
+    // cache line with the work counter, and a store per chunk took 50M double
+    // points from 1.1 to 2.3 ms.
     const unsigned long long corner = term + __shfl_down_sync(FULL, term, 1) + __shfl_down_sync(FULL, term, 2);
     if (lane == 0 && corner > 0x7FFFFFFFull && sm.overflowed != a.ctl) {
       a.ctl->id_overflow = 1u;
@@ -739,27 +812,17 @@ __device__ __forceinline__ uint32_t encode_chunk(const CArgs<T> &a, unsigned lon
   uint32_t bound;  // no block id is above it
   {
     T v[DIM][kEncPer];
-    load_points<T, DIM>(a, base, nvalid, v);
+    load_points<T, DIM>(a.x, a.y, a.z, base, nvalid, v);
     // bucket counts (last used as run starts, done with before the last chunk's planes)
     *reinterpret_cast<uint4 *>(H + 8 * t) = make_uint4(0u, 0u, 0u, 0u);
     *reinterpret_cast<uint4 *>(H + 8 * t + 4) = make_uint4(0u, 0u, 0u, 0u);
     if (t == 0) sm.ncrowd = 0u;
     // NaNs are ignored and -0.0 orders below +0.0, as in the reference's warp
     // reductions (:122-139); slots past the end repeat a point
-    T mn[3], mx[3];
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) warp_minmax(v[d], mn[d], mx[d]);
-    if (lane == 0) {
-      T *const m = reinterpret_cast<T *>(sm.mm[warp]);
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) {
-        m[d] = mn[d];
-        m[4 + d] = mx[d];
-      }
-    }
+    put_minmax<T, DIM>(sm, v, lane, warp);
     __syncthreads();  // 1: minima and maxima, the oldest parked payload's offset
     pending = pk.count == (uint32_t)kEncSlots;
-    if (warp == 0) chunk_scalars<T, DIM>(a, c, sm, seg, sh, eb, inv, lane);
+    if (warp == 0) encode_scalars<T, DIM>(a, c, sm, seg, sh, eb, inv, lane);
     else if (warp == kEncWarps - 1 && pending) look_up<T>(pa[pk.head], pk.head, sm, false, lane);
     __syncthreads();  // 2: the chunk's scalars
 
@@ -816,30 +879,8 @@ __device__ __forceinline__ uint32_t encode_chunk(const CArgs<T> &a, unsigned lon
   }
 
   // ---- 2. rank the composites (block id, r) ----
-  const bool narrow = bound < (1u << 22);
-  int how = 0;  // 0: radix, 1: narrow buckets, 2: wide buckets
-  if (full && bound >= (1u << kEncBucketBits) && rank_skip == 0u) {
-    if (narrow) how = rank_buckets<T, true>(sm, H, S, key, bound, t, lane, warp) ? 1 : 0;
-    else how = rank_buckets<T, false>(sm, H, S, key, bound, t, lane, warp) ? 2 : 0;
-    // one crowded bucket says little about the next chunk (a shuffled, clustered
-    // snapshot has a few); a second one in a row does (ordered points)
-    if (how != 0) declined = 0u;
-    else if (++declined >= 2u) rank_skip = kEncBucketBackoff;
-  } else if (rank_skip != 0u) {
-    --rank_skip;
-  }
-  const uint16_t *ranks = reinterpret_cast<const uint16_t *>(sm.Q);
-  if (how == 0) {
-    const uint32_t rbase = Points<T>::rank_base(t);
-    if (!full) {  // slots past the end sort last
-#pragma unroll
-      for (int e = 0; e < kEncPer; ++e)
-        if (Points<T>::point(t, e) >= nvalid) key[e] = bound + 1u;
-    }
-#pragma unroll
-    for (int e = 0; e < kEncPer; ++e) S[rx(rbase + Points<T>::rank_step(e))] = key[e];
-    ranks = radix_rank(S, H, reinterpret_cast<uint16_t *>(sm.Q), sm.tot, bitlen(bound + (full ? 0u : 1u)));
-  }
+  const uint16_t *ranks;
+  const int how = rank_chunk<T>(sm, H, S, key, bound, nvalid, rank_skip, declined, t, lane, warp, ranks);
 
   // ---- 3. runs: unique ids, deltas, counts (:222-311) ----
   // thread t takes positions 128j + t, so that neighbouring lanes hold

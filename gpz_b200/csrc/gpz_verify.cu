@@ -7,9 +7,8 @@
 // order (sorted by block within each chunk).  Here the pairing is recovered
 // exactly: for each 1024-point chunk the kernel recomputes what the encoder
 // sorted -- the composite (block id - min block id) << 10 | r, r being the
-// point's rank in the encoder's input order -- and sorts it, so sorted
-// position s of the chunk holds the composite of the point the decoder wrote
-// at s.  Every point is then checked against the bound, and per axis the
+// point's rank in the encoder's input order -- and ranks it, so sorted
+// position s of the chunk names the point the decoder wrote at s.  Every point is then checked against the bound, and per axis the
 // maximum error and the squared-error sum (for MSE / PSNR) are accumulated.
 // The quantization arithmetic is the compress kernel's (gpz_encode.cuh step
 // 1) so the block ids are the encoder's bit for bit.
@@ -20,7 +19,7 @@
 #include <cstring>
 
 #include "gpz_b200.h"
-#include "gpz_kernels.cuh"
+#include "gpz_encode.cuh"
 #include "gpz_launch.h"
 
 using namespace gpzb;
@@ -35,142 +34,156 @@ struct VerifyAcc {
   unsigned long long mm[6];     // ordered min (inverted) / max of the originals, per axis
 };
 
-constexpr int kVerifyWarps = 8;
+// Shared memory of a verify CTA: the ranking's, and the CTA's sums.
+struct VerifyShared : RankShared {
+  double sq[3][kEncWarps];
+  uint32_t over[kEncWarps], over_tol[kEncWarps];
+  unsigned long long emax[3][kEncWarps];
+  unsigned long long mn[3], mx[3];  // ordered minimum (inverted) / maximum of the chunks so far
+};
+constexpr int kVerifyCtas = 6;  // resident CTAs per SM the registers are sized for
 
+// A CTA of four warps takes one chunk after another: it repeats the encoder's
+// block ids and ranking (the same code: gpz_encode.cuh), which says which point
+// the decoder wrote at each position, and compares axis by axis, the originals
+// taken from shared memory in ranked order.
+//
+// Bound by instruction issue like the encoder (the 24 bytes a point would take
+// a tenth of the time).  A warp per chunk with a bitonic network of 64-bit
+// composites in shared memory (55 steps of 16 exchanges a lane) took 238 us on
+// 4M float 3D points; this form 43 us.
 template <typename T, int DIM>
-__global__ void __launch_bounds__(32 * kVerifyWarps) verify_kernel(const T *__restrict__ x, const T *__restrict__ y,
-                                                                   const T *__restrict__ z, const T *__restrict__ rx,
-                                                                   const T *__restrict__ ry, const T *__restrict__ rz,
-                                                                   unsigned long long n, T eb, uint32_t seg,
-                                                                   T bound, VerifyAcc *acc) {
+__global__ void __launch_bounds__(kEncThreads, kVerifyCtas)
+    verify_kernel(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ z, const T *__restrict__ rx,
+                  const T *__restrict__ ry, const T *__restrict__ rz, unsigned long long n, T eb, uint32_t seg, T bound,
+                  VerifyAcc *acc) {
   using UO = typename TT<T>::U;
   constexpr bool is64 = sizeof(T) == 8;
   constexpr uint32_t FULL = 0xFFFFFFFFu;
-  extern __shared__ __align__(16) unsigned long long vsm[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long *const C = vsm + warp * kChunk;
-  const T *X[3] = {x, y, z};
-  const T *R[3] = {rx, ry, rz};
-  const uint32_t sh = (uint32_t)__ffs((int)seg) - 1u, msk = seg - 1u;
-  (void)msk;
+  extern __shared__ __align__(16) unsigned char verify_smem[];
+  VerifyShared &sm = *reinterpret_cast<VerifyShared *>(verify_smem);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const T *const X[3] = {x, y, z};
+  const T *const Y[3] = {rx, ry, rz};
+  const uint32_t sh = (uint32_t)__ffs((int)seg) - 1u;
   const T inv = is64 ? (T)__ddiv_rn(1.0, __dmul_rn(2.0, (double)eb)) : (T)__fdiv_rn(1.0f, __fmul_rn(2.0f, (float)eb));
   const unsigned long long G = (n + kChunk - 1) / kChunk;
-  unsigned long long over = 0, over_tol = 0;
   const T tol = (T)1.01f * bound;
+  uint32_t over = 0, over_tol = 0, rank_skip = 0, declined = 0;
   T emax[3] = {0, 0, 0};
   double sq[3] = {0.0, 0.0, 0.0};
-  UO gmn[3] = {0, 0, 0}, gmx[3] = {0, 0, 0};
-  for (unsigned long long c = (unsigned long long)blockIdx.x * kVerifyWarps + warp; c < G;
-       c += (unsigned long long)gridDim.x * kVerifyWarps) {
+  if (t < 3) sm.mn[t] = sm.mx[t] = 0ull;
+  for (unsigned long long c = blockIdx.x; c < G; c += gridDim.x) {
     const unsigned long long base = c * kChunk;
     const uint32_t nvalid = (uint32_t)min((unsigned long long)kChunk, n - base);
-    // ---- block ids exactly as encode_chunk computes them ----
-    uint32_t key[32];
-    unsigned long long bnx = 0, bny = 0;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      T v[32];
-      const T lim = is64 ? (T)DBL_MAX : (T)FLT_MAX;
-      T mn = lim, mx = -lim;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const uint32_t p = 32u * j + lane;
-        v[j] = p < nvalid ? X[d][base + p] : (T)0;
-        if (p < nvalid) { mn = fmin(mn, v[j]); mx = fmax(mx, v[j]); }
+    const bool full = nvalid == (uint32_t)kChunk;
+    uint32_t *const H = sm.A[0], *const S = sm.A[1];
+    // ---- block ids exactly as the encoder computes them ----
+    uint32_t key[kEncPer], bnd;
+    {
+      T v[DIM][kEncPer];
+      load_points<T, DIM>(x, y, z, base, nvalid, v);
+      __syncthreads();  // the previous chunk's arrays have been read
+      *reinterpret_cast<uint4 *>(H + 8 * t) = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4 *>(H + 8 * t + 4) = make_uint4(0u, 0u, 0u, 0u);
+      if (t == 0) sm.ncrowd = 0u;
+      put_minmax<T, DIM>(sm, v, lane, warp);
+      __syncthreads();
+      if (warp == 0) {
+        unsigned long long term;
+        bool wide;
+        const T mmv = chunk_scalars<T, DIM>(sm, seg, sh, eb, inv, lane, term, wide);
+        if (lane < DIM) sm.mn[lane] = max(sm.mn[lane], (unsigned long long)(UO)~ord_of(mmv));
+        if (lane >= 3 && lane < 3 + DIM) sm.mx[lane - 3] = max(sm.mx[lane - 3], (unsigned long long)ord_of(mmv));
       }
-      mn = from_ord((UO)~warp_max((UO)~ord_of(mn)));
-      mx = from_ord(warp_max(ord_of(mx)));
-      gmn[d] = max(gmn[d], (UO)~ord_of(mn));
-      gmx[d] = max(gmx[d], ord_of(mx));
-      const T range = is64 ? (T)__dsub_rn((double)mx, (double)mn) : (T)__fsub_rn((float)mx, (float)mn);
-      if (d == 0) bnx = block_num(range, seg, eb, is64 && DIM == 2);
-      if (d == 1) bny = block_num(range, seg, eb, false);
-      const T nmn = is64 ? (T)__dmul_rn(-(double)mn, (double)inv) : (T)__fmul_rn(-(float)mn, (float)inv);
-      const uint32_t kmul = d == 0 ? 1u : (d == 1 ? (uint32_t)bnx : (uint32_t)(bnx * bny));
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        uint32_t kq;
-        if constexpr (!is64) {
-          kq = __float2uint_rz(__fmaf_rn((float)v[j], (float)inv, (float)nmn)) >> sh;
-        } else {
-          kq = (uint32_t)(__double2ull_rz(__fma_rn((double)v[j], (double)inv, (double)nmn)) >> sh);
-        }
-        key[j] = d == 0 ? kq : key[j] + kq * kmul;
-      }
-    }
-    uint32_t kmin = FULL;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      key[j] &= 0x7FFFFFFFu;
-      if (32u * j + lane < nvalid) kmin = min(kmin, key[j]);
-    }
-    kmin = warp_min(kmin);
-    // composites: point p = 32j + lane has rank r = 32 lane + j
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const uint32_t r = 32u * lane + j;
-      C[r] = 32u * j + lane < nvalid ? ((unsigned long long)(key[j] - kmin) << 10) | r : ~0ull;
-    }
-    __syncwarp();
-    // ---- ascending bitonic sort of the 1024 composites in shared memory ----
-    for (uint32_t k = 2; k <= (uint32_t)kChunk; k <<= 1) {
-      for (uint32_t jj = k >> 1; jj > 0; jj >>= 1) {
-        for (uint32_t q = lane; q < (uint32_t)kChunk / 2; q += 32) {
-          const uint32_t i = ((q & ~(jj - 1)) << 1) | (q & (jj - 1));
-          const uint32_t p = i + jj;
-          const bool up = (i & k) == 0;
-          const unsigned long long a = C[i], b = C[p];
-          if ((a > b) == up) {
-            C[i] = b;
-            C[p] = a;
-          }
-        }
-        __syncwarp();
-      }
-    }
-    // ---- sorted position s holds the point the decoder wrote at s ----
-#pragma unroll 4
-    for (int j = 0; j < 32; ++j) {
-      const uint32_t s = 32u * j + lane;
-      if (s >= nvalid) continue;
-      const uint32_t r = (uint32_t)(C[s] & 1023u);
-      const uint32_t p = (r & 31u) * 32u + (r >> 5);
-      bool off = false, off_tol = false;
+      __syncthreads();
+      const uint4 sc = ld4(sm.sc);
+      bnd = sc.z;
 #pragma unroll
       for (int d = 0; d < DIM; ++d) {
-        const T o = X[d][base + p], rec = R[d][base + s];
-        const T e = o > rec ? o - rec : rec - o;
-        off |= !(e <= bound);
-        off_tol |= !(e <= tol);
+        const T nmd = reinterpret_cast<const T *>(sm.nm)[d];
+        const uint32_t kmul = d == 1 ? sc.x : sc.y;
+#pragma unroll
+        for (int e = 0; e < kEncPer; ++e) {
+          uint32_t kq;
+          if constexpr (!is64) kq = __float2uint_rz(__fmaf_rn((float)v[d][e], (float)inv, (float)nmd)) >> sh;
+          else kq = (uint32_t)(__double2ull_rz(__fma_rn((double)v[d][e], (double)inv, (double)nmd)) >> sh);
+          key[e] = d == 0 ? kq : key[e] + kq * kmul;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < kEncPer; ++e) key[e] &= 0x7FFFFFFFu;
+    }
+    // ---- the order the encoder gave them ----
+    const uint16_t *ranks;
+    const int how = rank_chunk<T>(sm, H, S, key, bnd, nvalid, rank_skip, declined, t, lane, warp, ranks);
+    uint32_t r[8];  // point at position 128j + t
+#pragma unroll
+    for (int j = 0; j < 8; ++j) r[j] = point_of_rank(how == 1 ? H[128 * j + t] & 1023u : (uint32_t)ranks[128 * j + t]);
+    __syncthreads();  // the ranking's arrays are free
+    // ---- position s holds the point the decoder wrote at s ----
+    uint32_t off = 0, off_tol = 0;  // bit j: position 128j + t is off on some axis
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      // the axis by point, in one of two 8 KB halves in turn
+      T *const O = reinterpret_cast<T *>(d & 1 ? sm.R : sm.A[0]);
+      {
+        T v[1][kEncPer];
+        load_points<T, 1>(X[d], X[d], X[d], base, nvalid, v);
+#pragma unroll
+        for (int e = 0; e < kEncPer; ++e) O[Points<T>::point(t, e)] = v[0][e];
+      }
+      T rec[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) rec[j] = full || 128u * j + t < nvalid ? Y[d][base + 128u * j + t] : (T)0;
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (!full && 128u * j + t >= nvalid) continue;
+        const T o = O[r[j]];
+        const T e = o > rec[j] ? o - rec[j] : rec[j] - o;
+        if (!(e <= bound)) off |= 1u << j;
+        if (!(e <= tol)) off_tol |= 1u << j;
         emax[d] = fmax(emax[d], e);
         sq[d] += (double)e * (double)e;
       }
-      over += off ? 1ull : 0ull;
-      over_tol += off_tol ? 1ull : 0ull;
     }
-    __syncwarp();
+    over += __popc(off);
+    over_tol += __popc(off_tol);
   }
-  // ---- warp, then global accumulation ----
-  over = __reduce_add_sync(FULL, (uint32_t)over);
-  over_tol = __reduce_add_sync(FULL, (uint32_t)over_tol);
+  // ---- CTA sums, then one atomic per value and CTA ----
+  over = __reduce_add_sync(FULL, over);
+  over_tol = __reduce_add_sync(FULL, over_tol);
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
     const UO em = warp_max(ord_of(emax[d]));
     double s = sq[d];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-    const UO a = warp_max(gmn[d]), b = warp_max(gmx[d]);
     if (lane == 0) {
-      atomicMax(&acc->max_err[d], (unsigned long long)em);
-      atomicAdd(&acc->sq[d], s);
-      atomicMax(&acc->mm[2 * d], (unsigned long long)a);
-      atomicMax(&acc->mm[2 * d + 1], (unsigned long long)b);
+      sm.emax[d][warp] = (unsigned long long)em;
+      sm.sq[d][warp] = s;
     }
   }
   if (lane == 0) {
-    atomicAdd(&acc->over, over);
-    atomicAdd(&acc->over_tol, over_tol);
+    sm.over[warp] = over;
+    sm.over_tol[warp] = over_tol;
   }
+  __syncthreads();
+  if (t < DIM) {
+    unsigned long long em = 0;
+    double s = 0.0;
+    for (int w = 0; w < kEncWarps; ++w) {
+      em = max(em, sm.emax[t][w]);
+      s += sm.sq[t][w];
+    }
+    atomicMax(&acc->max_err[t], em);
+    atomicAdd(&acc->sq[t], s);
+    atomicMax(&acc->mm[2 * t], sm.mn[t]);
+    atomicMax(&acc->mm[2 * t + 1], sm.mx[t]);
+  }
+  if (t == 32) atomicAdd(&acc->over, (unsigned long long)sm.over[0] + sm.over[1] + sm.over[2] + sm.over[3]);
+  if (t == 33) atomicAdd(&acc->over_tol, (unsigned long long)sm.over_tol[0] + sm.over_tol[1] + sm.over_tol[2] + sm.over_tol[3]);
 }
 
 template <typename T>
@@ -185,16 +198,16 @@ int verify_t(uint32_t dim, uint64_t n, const void *dx, const void *dy, const voi
              cudaStream_t st) {
   VerifyAcc *acc = static_cast<VerifyAcc *>(d_scratch);
   if (cudaMemsetAsync(acc, 0, sizeof(VerifyAcc), st) != cudaSuccess) return GPZ_ECUDA;
-  const size_t smem = (size_t)kVerifyWarps * kChunk * 8;
+  const size_t smem = sizeof(VerifyShared);
   const T *x = (const T *)dx, *y = (const T *)dy, *z = (const T *)(dim == 3 ? dz : dy);
   const T *a = (const T *)rx, *b = (const T *)ry, *c = (const T *)(dim == 3 ? rz : ry);
   const int sms = current_sms();
   const uint64_t G = (n + kChunk - 1) / kChunk;
   auto launch = [&](auto kernel) -> bool {
-    const int occ = resident_ctas(kernel, 32 * kVerifyWarps, smem);
+    const int occ = resident_ctas(kernel, kEncThreads, smem);
     if (occ == 0) return false;
-    const uint64_t grid = std::min<uint64_t>((G + kVerifyWarps - 1) / kVerifyWarps, (uint64_t)sms * occ);
-    kernel<<<(unsigned)grid, 32 * kVerifyWarps, smem, st>>>(x, y, z, a, b, c, n, (T)eb, seg, (T)bound, acc);
+    const uint64_t grid = std::min<uint64_t>(G, (uint64_t)sms * occ);
+    kernel<<<(unsigned)grid, kEncThreads, smem, st>>>(x, y, z, a, b, c, n, (T)eb, seg, (T)bound, acc);
     return true;
   };
   if (!(dim == 3 ? launch(verify_kernel<T, 3>) : launch(verify_kernel<T, 2>))) return GPZ_ECUDA;
