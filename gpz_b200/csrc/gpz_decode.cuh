@@ -94,58 +94,71 @@ __device__ __forceinline__ uint32_t bplane_lo(const uint32_t *__restrict__ pw, u
 // Bytes 4*lane..4*lane+3 of the plane as a word in element order (bit t =
 // element 32*lane + t), masked to the lane's valid elements `vm`.  The
 // unaligned window takes its upper part from the next lane's aligned word;
-// lane 31 loads its own when the plane is longer than 124 bytes.
-__device__ __forceinline__ uint32_t bplane_word(uint32_t lo, const uint32_t *__restrict__ pw, uint32_t pos,
-                                                uint32_t bpp, uint32_t endw, uint32_t vm, int lane) {
+// lane 31's, when the plane is longer than 124 bytes, is a word of the plane
+// behind: `after` holds that plane's aligned words (or, for the section's last
+// plane, just that word in lane 31).
+template <bool LAST>
+__device__ __forceinline__ uint32_t bplane_word(uint32_t lo, uint32_t after, uint32_t pos, uint32_t bpp, uint32_t vm,
+                                                int lane) {
   uint32_t hi = __shfl_down_sync(0xFFFFFFFFu, lo, 1);
   if (bpp > 124u) {
-    const uint32_t a32 = (pos >> 2) + 32u;
-    if (lane == 31) hi = a32 < endw ? __ldg(pw + a32) : 0u;
+    const uint32_t h = LAST ? after : __shfl_sync(0xFFFFFFFFu, after, (int)((pos >> 2) + 32u - ((pos + bpp) >> 2)));
+    if (lane == 31) hi = h;
   }
   return from_msb_bytes(__funnelshift_r(lo, hi, (pos & 3u) << 3)) & vm;
 }
 
-// Plane words of one section loaded ahead of use (when it has at most CAP
-// planes): w[b] = the aligned word of value bit b's plane.
+// Aligned words of one section's low CAP planes, loaded ahead of use: w[b] =
+// value bit b's plane; `tail` in lane 31: the word behind the last plane's.
 template <int CAP, bool BYTES>
 struct PlaneWords {
   uint32_t w[CAP];
+  uint32_t tail;
+  __device__ __forceinline__ static uint32_t word(const uint32_t *__restrict__ pw, uint32_t pos0, uint32_t nb,
+                                                  uint32_t b, uint32_t bpp, uint32_t endw, int lane) {
+    if (b >= nb) return 0u;
+    const uint32_t pi = nb - 1u - b;
+    return BYTES ? bplane_lo(pw, pos0 + pi * bpp, endw, lane) : __ldg(pw + (pos0 >> 2) + 32u * pi + lane);
+  }
   __device__ __forceinline__ void load(const uint32_t *__restrict__ pw, uint32_t pos0, uint32_t nb, uint32_t bpp,
                                        uint32_t endw, int lane) {
-    const bool pre = nb <= (uint32_t)CAP;
-#pragma unroll
-    for (int b = 0; b < CAP; ++b) {
-      w[b] = 0u;
-      if (pre && (uint32_t)b < nb) {
-        const uint32_t pi = nb - 1u - b;
-        w[b] = BYTES ? bplane_lo(pw, pos0 + pi * bpp, endw, lane) : __ldg(pw + (pos0 >> 2) + 32u * pi + lane);
-      }
+    if constexpr (BYTES) {
+      const uint32_t at = ((pos0 + (nb - 1u) * bpp) >> 2) + 32u;
+      tail = nb != 0u && bpp > 124u && lane == 31 && at < endw ? __ldg(pw + at) : 0u;
     }
+#pragma unroll
+    for (int b = 0; b < CAP; ++b) w[b] = word(pw, pos0, nb, b, bpp, endw, lane);
   }
 };
 
 // This lane's transposed section words: N = 8 gives quads (value k | k+8 <<
 // 8 | k+16 << 16 | k+24 << 24), N = 16 pairs (value k | k+16 << 16), N = 32
-// values.  Requires nb <= N; planes come from `raw` when N <= CAP.  `orw`
-// collects the OR of the (masked) plane words.
+// values.  Requires nb <= N; the low CAP planes come from `raw`, the others are
+// loaded here, all in flight at once before the first is used (one load per
+// plane in turn made sections of more than 16 planes -- double lattices, tight
+// bounds -- a chain of up to 16 load latencies).  `orw` collects the OR of the
+// (masked) plane words.
 template <int N, int CAP, bool BYTES>
 __device__ __forceinline__ void section_words(uint32_t (&q)[N], const PlaneWords<CAP, BYTES> &raw,
                                               const uint32_t *__restrict__ pw, uint32_t pos0, uint32_t nb,
                                               uint32_t bpp, uint32_t endw, uint32_t vm, int lane, uint32_t &orw) {
 #pragma unroll
-  for (int b = 0; b < N; ++b) {
-    uint32_t w = 0u;
-    if ((uint32_t)b < nb) {
-      const uint32_t pi = nb - 1u - b;
-      const uint32_t pos = pos0 + pi * bpp;
-      uint32_t lo;
-      if constexpr (N <= CAP) lo = raw.w[b < CAP ? b : 0];
-      else lo = BYTES ? bplane_lo(pw, pos, endw, lane) : __ldg(pw + (pos0 >> 2) + 32u * pi + lane);
-      w = BYTES ? bplane_word(lo, pw, pos, bpp, endw, vm, lane) : lo;
+  for (int b = 0; b < N; ++b)
+    q[b] = b < CAP ? raw.w[b < CAP ? b : 0] : PlaneWords<CAP, BYTES>::word(pw, pos0, nb, b, bpp, endw, lane);
+  if constexpr (BYTES) {
+    // top plane first: each takes the word behind it from the plane below,
+    // whose words are still as loaded
+#pragma unroll
+    for (int b = N - 1; b >= 0; --b) {
+      if ((uint32_t)b < nb) {
+        const uint32_t pos = pos0 + (nb - 1u - b) * bpp;
+        q[b] = b == 0 ? bplane_word<true>(q[0], raw.tail, pos, bpp, vm, lane)
+                      : bplane_word<false>(q[b], q[b > 0 ? b - 1 : 0], pos, bpp, vm, lane);
+      }
     }
-    q[b] = w;
-    orw |= w;
   }
+#pragma unroll
+  for (int b = 0; b < N; ++b) orw |= q[b];
   if constexpr (N == 8) planes8_to_quads(q);
   else if constexpr (N == 16) planes16_to_pairs(q);
   else transpose32(q);
