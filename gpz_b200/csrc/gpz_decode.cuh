@@ -192,13 +192,21 @@ __device__ __forceinline__ uint32_t rel_coord(uint32_t rp, const ChunkGeom &g) {
   return (2u * g.sh >= 32u) ? 0u : (rp >> (2u * g.sh));
 }
 
-template <typename T>
+// kSmall (double): the quantized value is below 2^31, so 2q + 1 becomes a double
+// exactly through the mantissa of 2^52, without a 64-bit conversion.
+template <typename T, bool kSmall>
 __device__ __forceinline__ uint32_t value_bits(unsigned long long b, uint32_t rel, uint32_t seg, T eb, T mn,
                                                uint32_t &hi) {
   if constexpr (sizeof(T) == 4) {
     const uint32_t q = (uint32_t)b * seg + rel;
     hi = 0u;
     return __float_as_uint(__fmaf_rn(__uint2float_rn((q << 1) | 1u), (float)eb, (float)mn));
+  } else if constexpr (kSmall) {
+    const uint32_t q = (uint32_t)b * seg + rel;
+    const double d = __dadd_rn(__hiloint2double(0x43300000, (int)((q << 1) | 1u)), -4503599627370496.0);
+    const double v = __fma_rn(d, (double)eb, (double)mn);
+    hi = (uint32_t)__double2hiint(v);
+    return (uint32_t)__double2loint(v);
   } else {
     const unsigned long long q = b * (unsigned long long)seg + rel;
     const unsigned long long v =
@@ -234,8 +242,70 @@ __device__ __forceinline__ void copy_out_rows(const uint32_t *stage, T *dst, int
   }
 }
 
+// All axes of a float chunk with ids below 2^31, one pass over the positions: a
+// lane takes its quads of ids and relative positions once, and twice the
+// quantized value plus one is formed directly (modulo 2^32),
+//   2 q + 1 = b * 2 seg + ((2 rel part) | 1);
+// axis x replaces the ids, y the relative positions, z goes to C, all in the
+// lane's own quads, and three coalesced copies follow.
+//
+// Bound by instruction issue.  One pass per axis, the quotients written back
+// between them, took 3.83 K instructions and 813 shared wavefronts a chunk and
+// 0.76 ms on the 143.7M-point snapshot; this form 3.58 K, 610 and 0.73 ms.  For
+// doubles the same form (a quarter of the positions at a time, for room) was
+// slower, 458 against 420 us on 50M lattice points: bank conflicts and twice
+// the code.
+struct FastGeom {
+  uint32_t seg2, msk2, ysh, zsh;
+  __device__ __forceinline__ explicit FastGeom(const ChunkGeom &g)
+      : seg2(2u * g.seg), msk2(2u * g.msk), ysh(g.sh), zsh(2u * g.sh < 32u ? 2u * g.sh : 31u) {}
+};
+
+// 2 q + 1 on every axis of the point with id n and relative position rp.
+template <int DIM>
+__device__ __forceinline__ void odd_values(uint32_t n, uint32_t rp, const ChunkGeom &g, const FastGeom &f,
+                                           uint32_t (&v)[3]) {
+  const uint32_t r2 = rp << 1;
+  const uint32_t q1 = g.gx.div2(n + n), q2 = g.gy.div2(q1 + q1);
+  v[0] = (n - q1 * g.bnx) * f.seg2 + ((r2 & f.msk2) | 1u);
+  v[1] = (q1 - q2 * g.bny) * f.seg2 + (((r2 >> f.ysh) & f.msk2) | 1u);
+  v[2] = DIM == 3 ? q2 * f.seg2 + ((r2 >> f.zsh) | 1u) : 0u;
+}
+
+template <int DIM, class Cfg>
+__device__ __forceinline__ void reconstruct_all(uint32_t *sw, const ChunkGeom &g, float eb, const float (&mm)[6],
+                                                float *const (&Y)[3], unsigned long long base, int lane,
+                                                uint32_t nvalid, bool full) {
+  const FastGeom f(g);
+  uint32_t *const P = sw + Cfg::P, *const R = sw + Cfg::R, *const C = sw + Cfg::C;
+#pragma unroll 1
+  for (int m = 0; m < 8; ++m) {
+    const uint32_t at = qoff(lane, m);
+    const uint4 p4 = *reinterpret_cast<const uint4 *>(P + at), r4 = *reinterpret_cast<const uint4 *>(R + at);
+    const uint32_t pp[4] = {p4.x, p4.y, p4.z, p4.w}, rr[4] = {r4.x, r4.y, r4.z, r4.w};
+    uint32_t o[3][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      uint32_t v[3];
+      odd_values<DIM>(pp[e], rr[e], g, f, v);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) o[d][e] = __float_as_uint(__fmaf_rn(__uint2float_rn(v[d]), eb, mm[d]));
+    }
+    *reinterpret_cast<uint4 *>(P + at) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
+    *reinterpret_cast<uint4 *>(R + at) = make_uint4(o[1][0], o[1][1], o[1][2], o[1][3]);
+    if (DIM == 3) *reinterpret_cast<uint4 *>(C + at) = make_uint4(o[2][0], o[2][1], o[2][2], o[2][3]);
+  }
+  __syncwarp();
+  copy_out_rows<float>(P, Y[0] + base, lane, 0u, nvalid, full);
+  copy_out_rows<float>(R, Y[1] + base, lane, 0u, nvalid, full);
+  if (DIM == 3) copy_out_rows<float>(C, Y[2] + base, lane, 0u, nvalid, full);
+  __syncwarp();
+}
+
 // One axis.  MODE 0: P holds ids (axis 0), then id/bnx (axis 1), then
-// id/(bnx*bny) (axis 2), each axis leaving the next quotient in place.
+// id/(bnx*bny) (axis 2), each axis leaving the next quotient in place, and
+// the quantized values are below 2^31 (float chunks go through
+// reconstruct_all instead).  MODE 3: the same without the limit.
 // MODE 1: P holds 32-bit ids, general dividers.  MODE 2 (double streams): P
 // holds run indices, 64-bit ids come from the id table.
 template <typename T, int D, int MODE, bool KEEP, class Cfg>
@@ -258,7 +328,7 @@ __device__ __forceinline__ void reconstruct_axis(uint32_t *sw, const ChunkGeom &
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         unsigned long long b;
-        if constexpr (MODE == 0) {
+        if constexpr (MODE == 0 || MODE == 3) {
           const uint32_t n = pp[e];
           if constexpr (D == 2) {
             b = n;
@@ -283,9 +353,9 @@ __device__ __forceinline__ void reconstruct_axis(uint32_t *sw, const ChunkGeom &
             else b = dxy ? id / dxy : ~0ull;
           }
         }
-        lo[e] = value_bits<T>(b, rel_coord<D>(rr[e], g), g.seg, eb, mn, hi[e]);
+        lo[e] = value_bits<T, MODE == 0>(b, rel_coord<D>(rr[e], g), g.seg, eb, mn, hi[e]);
       }
-      if constexpr (MODE == 0 && D < 2 && KEEP)
+      if constexpr ((MODE == 0 || MODE == 3) && D < 2 && KEEP)
         *reinterpret_cast<uint4 *>(P + qoff(lane, mq)) = make_uint4(nq[0], nq[1], nq[2], nq[3]);
       if constexpr (!is64) {
         *reinterpret_cast<uint4 *>(C + qoff(lane, m)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -502,7 +572,7 @@ __device__ __forceinline__ void decode_chunk(const DArgs<T> &a, unsigned long lo
   __syncwarp();  // run map rows cleared
 
   // ---- deltas -> ids: id[0] = first, id[u] = id[u-1] + delta[u] (:930-938) ----
-  bool fast = false, bail = false;
+  bool fast = false, bail = false, small = false;
   {
     auto run_ids = [&](auto &q) {
       constexpr int N = sizeof(q) / sizeof(uint32_t);
@@ -533,6 +603,13 @@ __device__ __forceinline__ void decode_chunk(const DArgs<T> &a, unsigned long lo
       // bits.  (A corrupt stream can only yield wrong coordinates here, no
       // access depends on the ids.)
       const unsigned long long total = (unsigned long long)__shfl_sync(FULL, inc, 31);
+      if (is64) {
+        // every axis's quantized values below 2^31: block counts of x and y, the
+        // largest id's z block (floats rounded, hence the lower limit)
+        const float zb = (float)(first + total) / (float)max(bnx * bny, 1ull);
+        small = bnx * (unsigned long long)seg < (1ull << 31) && bny * (unsigned long long)seg < (1ull << 31) &&
+                (zb + 2.0f) * (float)seg < 2.0e9f;
+      }
       fast = first + total < (1ull << 31) && !g.wide && bnx != 0 && bny != 0 && bnx * bny < (1ull << 32);
       if constexpr (PASS == kPassFast) {
         // the fast layout has no id tables: ids of 2^31 or more (which no
@@ -631,7 +708,9 @@ __device__ __forceinline__ void decode_chunk(const DArgs<T> &a, unsigned long lo
   // ---- reconstruct ----
   const bool full = nvalid == (uint32_t)kChunk && a.vec_ok;
   if (fast) {
-    reconstruct<T, DIM, 0, Cfg>(sw, g, eb, mm, Y, base, lane, nvalid, full);
+    if constexpr (!is64) reconstruct_all<DIM, Cfg>(sw, g, eb, mm, Y, base, lane, nvalid, full);
+    else if (small) reconstruct<T, DIM, 0, Cfg>(sw, g, eb, mm, Y, base, lane, nvalid, full);
+    else reconstruct<T, DIM, 3, Cfg>(sw, g, eb, mm, Y, base, lane, nvalid, full);
   } else {
     FastDiv f;
     f.init(my_div);

@@ -53,3 +53,18 @@ def test_relative_position_widths(bits, seg):
     got = gz.decompress(torch.from_numpy(np.frombuffer(s, np.uint8).copy()).cuda())
     for a, b in zip(got, want):
         assert np.array_equal(a.cpu().numpy(), b)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e3, 1e6])
+@pytest.mark.parametrize("flat", [0, 1])
+def test_double_quantized_values_around_2_to_the_31(scale, flat):
+    """Double 2D chunks whose quantized values pass 2^31 on one axis while the block counts' product stays in 32 bits."""
+    rng = np.random.default_rng(int(scale) + flat)
+    n = 2 * 1024 + 5
+    long = rng.random(n) * 1500.0 * scale
+    short = rng.random(n) * 1e-3
+    x, y = (short, long) if flat else (long, short)
+    s = po.compress(x, y, np.zeros_like(x), 2, 2.5e-4, 64)
+    ox, oy, _ = po.decompress(s)
+    dx, dy, _ = gz.decompress(torch.from_numpy(np.frombuffer(s, np.uint8).copy()).cuda())
+    assert np.array_equal(dx.cpu().numpy(), ox) and np.array_equal(dy.cpu().numpy(), oy)
