@@ -50,9 +50,11 @@ bool decompress_layout(const gpz_dbatch_item *items, uint32_t count, Layout &L);
 void compress_tables(const gpz_batch_item *items, const Layout &L, uint8_t *dev, uint8_t *image);
 void decompress_tables(const gpz_dbatch_item *items, const Layout &L, uint8_t *dev, uint8_t *image);
 
-// Clears the control range and launches the class kernels on `st`.
-void compress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st);
-void decompress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st);
+// Clears the control range and launches the class kernels on `st`: one class
+// after another, or, with `branches` on a capturing stream, as parallel
+// branches of the graph.
+void compress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st, bool branches = false);
+void decompress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st, bool branches = false);
 
 // Item i's control block (compress: also its rel->abs block at count + i).
 inline uint64_t ctl_off(uint32_t i) { return (uint64_t)i * 256u; }

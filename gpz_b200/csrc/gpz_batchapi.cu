@@ -3,13 +3,14 @@
 // include/gpz_b200.h (gpz_batch_*, gpz_dbatch_*), which captures them in a
 // CUDA graph.
 //
-// Classes are (float, 2D), (float, 3D), (double, 2D), (double, 3D); a batch
-// runs them one after another: (compress) rel->abs when any of its snapshots
-// asks for it, sampling, one persistent compress kernel; (decompress) a header
-// check per stream, one persistent decompress kernel.  Two different codec
-// kernels resident on one SM thrash its instruction cache (each is a few
-// hundred KB of unrolled code), which costs far more than overlapping the
-// classes would gain.
+// Classes are (float, 2D), (float, 3D), (double, 2D), (double, 3D): (compress)
+// rel->abs when any of its snapshots asks for it, sampling, one persistent
+// compress kernel; (decompress) a header check per stream, one persistent
+// decompress kernel.  A plan's graph runs its classes as parallel branches, so
+// that a class's launches and last chunks overlap the others' work: 368 -> 294
+// us for 48 mixed snapshots of 10,000 to 1.2M points, 137 -> 64 us for 16 of
+// 1,600 to 200,000.  The server's batches run them one after another on the
+// slot's stream.
 
 #include <algorithm>
 #include <cstring>
@@ -127,6 +128,42 @@ void enqueue_dclass(const gpzb_host::ClassPlan &cp, uint8_t *dev, cudaStream_t s
         <<<cp.grid2, 32 * DecCfg<T>::warps, dec_smem_bytes<T>(), st>>>(tab, map, cp.work);
   }
 }
+
+// Parallel branches on one capturing stream: each begin() goes back to the
+// nodes captured before the first branch, join() makes what follows wait for
+// all of them.  Does nothing when `on` is not set; a failing call invalidates
+// the capture, which its end reports.
+class CaptureBranches {
+ public:
+  CaptureBranches(cudaStream_t st, bool on) : st_(st), on_(on) {
+    if (on_) root_ = nodes();
+  }
+  void begin() {
+    if (on_) cudaStreamUpdateCaptureDependencies(st_, root_.data(), root_.size(), cudaStreamSetCaptureDependencies);
+  }
+  void end() {
+    if (!on_) return;
+    const std::vector<cudaGraphNode_t> n = nodes();
+    ends_.insert(ends_.end(), n.begin(), n.end());
+  }
+  void join() {
+    if (on_) cudaStreamUpdateCaptureDependencies(st_, ends_.data(), ends_.size(), cudaStreamSetCaptureDependencies);
+  }
+
+ private:
+  std::vector<cudaGraphNode_t> nodes() const {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t *deps = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo(st_, &status, nullptr, nullptr, &deps, &n) != cudaSuccess ||
+        status != cudaStreamCaptureStatusActive)
+      n = 0;
+    return std::vector<cudaGraphNode_t>(deps, deps + n);
+  }
+  cudaStream_t st_;
+  bool on_;
+  std::vector<cudaGraphNode_t> root_, ends_;
+};
 
 }  // namespace
 
@@ -260,31 +297,39 @@ void decompress_tables(const gpz_dbatch_item *items, const Layout &L, uint8_t *d
   }
 }
 
-void compress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st) {
+void compress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st, bool branches) {
   cudaMemsetAsync(dev, 0, L.zero_bytes, st);
+  CaptureBranches br(st, branches);
   for (int c = 0; c < 4; ++c) {
     if (L.cls[c].items.empty()) continue;
     const uint64_t claim = L.claim_off + 8ull * c;
+    br.begin();
     switch (c) {
       case 0: enqueue_class<float, 2>(L.cls[c], L.count, dev, claim, st); break;
       case 1: enqueue_class<float, 3>(L.cls[c], L.count, dev, claim, st); break;
       case 2: enqueue_class<double, 2>(L.cls[c], L.count, dev, claim, st); break;
       default: enqueue_class<double, 3>(L.cls[c], L.count, dev, claim, st); break;
     }
+    br.end();
   }
+  br.join();
 }
 
-void decompress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st) {
+void decompress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st, bool branches) {
   cudaMemsetAsync(dev, 0, L.zero_bytes, st);
+  CaptureBranches br(st, branches);
   for (int c = 0; c < 4; ++c) {
     if (L.cls[c].items.empty()) continue;
+    br.begin();
     switch (c) {
       case 0: enqueue_dclass<float, 2>(L.cls[c], dev, st); break;
       case 1: enqueue_dclass<float, 3>(L.cls[c], dev, st); break;
       case 2: enqueue_dclass<double, 2>(L.cls[c], dev, st); break;
       default: enqueue_dclass<double, 3>(L.cls[c], dev, st); break;
     }
+    br.end();
   }
+  br.join();
 }
 
 }  // namespace gpzb_host
@@ -376,7 +421,7 @@ int gpz_batch_create(const gpz_batch_item *items, uint32_t count, gpz_batch **ba
   b->items.assign(items, items + count);
   const int rc = make_plan(
       b->plan, L, [&](uint8_t *dev, uint8_t *image) { gpzb_host::compress_tables(items, L, dev, image); },
-      [&](uint8_t *dev, cudaStream_t s) { gpzb_host::compress_enqueue(L, dev, s); });
+      [&](uint8_t *dev, cudaStream_t s) { gpzb_host::compress_enqueue(L, dev, s, true); });
   if (rc != GPZ_OK) {
     delete b;
     return rc;
@@ -434,7 +479,7 @@ int gpz_dbatch_create(const gpz_dbatch_item *items, uint32_t count, gpz_dbatch *
   if (!b) return GPZ_ECUDA;
   const int rc = make_plan(
       b->plan, L, [&](uint8_t *dev, uint8_t *image) { gpzb_host::decompress_tables(items, L, dev, image); },
-      [&](uint8_t *dev, cudaStream_t s) { gpzb_host::decompress_enqueue(L, dev, s); });
+      [&](uint8_t *dev, cudaStream_t s) { gpzb_host::decompress_enqueue(L, dev, s, true); });
   if (rc != GPZ_OK) {
     delete b;
     return rc;
