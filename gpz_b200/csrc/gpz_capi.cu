@@ -62,8 +62,9 @@ int compress_t(const gpz_params *p, const void *d_x, const void *d_y, const void
   Control *ctl = static_cast<Control *>(d_scratch);
   // the look-back records: the first in the control block, the others behind it
   unsigned long long *look = reinterpret_cast<unsigned long long *>(static_cast<uint8_t *>(d_scratch) + kLookTail);
-  cudaError_t e = cudaMemsetAsync(d_scratch, 0, kCtlBytes + look_bytes(G), st);
-  if (e != cudaSuccess) return GPZ_ECUDA;
+  // a small snapshot's sampling kernel clears the control block itself
+  const bool small = p->n <= kSmallPoints && !(p->flags & (GPZ_FLAG_SEG_FIXED | GPZ_FLAG_STRICT_BOUND));
+  if (!small && cudaMemsetAsync(d_scratch, 0, kCtlBytes + look_bytes(G), st) != cudaSuccess) return GPZ_ECUDA;
   const T eb = (T)p->eb;
   const T rel = (T)p->rel_eb;
   const T *x = static_cast<const T *>(d_x), *y = static_cast<const T *>(d_y), *z = static_cast<const T *>(d_z);
@@ -76,6 +77,10 @@ int compress_t(const gpz_params *p, const void *d_x, const void *d_y, const void
   if (p->flags & GPZ_FLAG_SEG_FIXED) {
     if (p->seg_size == 0) return GPZ_EINVAL;
     set_seg_kernel<<<1, 1, 0, st>>>(ctl, p->seg_size);
+  } else if (small) {
+    static_assert(kSmallPoints <= (uint64_t)kLookGroup * kChunk, "all look-back records in the control block");
+    seg_small_kernel<T><<<1, 1024, 0, st>>>(x, y, p->dim == 3 ? z : y, p->n, p->dim, p->seg_size, p->rel_mode, rel, eb,
+                                            (p->flags & GPZ_FLAG_SAFE31) ? 1 : 0, ctl);
   } else {
     const int safe31 = (p->flags & (GPZ_FLAG_SAFE31 | GPZ_FLAG_STRICT_BOUND)) ? 1 : 0;
     seg_sample_kernel<T><<<128, 256, 0, st>>>(x, y, p->dim == 3 ? z : y, p->n, p->dim, p->seg_size, p->rel_mode, rel,
@@ -323,19 +328,24 @@ int gpz_rel_to_abs(uint32_t float_bits, uint32_t dim, uint64_t n, const void *d_
   if (scratch_bytes < (uint64_t)kCtlBytes) return GPZ_ENOSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Control *ctl = static_cast<Control *>(d_scratch);
-  if (cudaMemsetAsync(d_scratch, 0, kCtlBytes, st) != cudaSuccess) return GPZ_ECUDA;
-  // enough blocks for the loads in flight, no more than the work fills
-  const uint64_t per_block = 256ull * kFoldUnroll * (float_bits == 32 ? 4 : 2);
-  const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)num_sms() * 6, (n + per_block - 1) / per_block));
-  if (float_bits == 32)
-    rel_to_abs_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float *>(d_x), static_cast<const float *>(d_y),
-                                                   static_cast<const float *>(dim == 3 ? d_z : d_y), n, dim,
-                                                   (float)rel, ctl);
-  else
-    rel_to_abs_kernel<double><<<grid, 256, 0, st>>>(static_cast<const double *>(d_x),
-                                                    static_cast<const double *>(d_y),
-                                                    static_cast<const double *>(dim == 3 ? d_z : d_y), n, dim, rel,
-                                                    ctl);
+  auto run = [&](auto zero, auto small_kernel, auto kernel) -> bool {
+    using T = decltype(zero);
+    const T *x = static_cast<const T *>(d_x), *y = static_cast<const T *>(d_y);
+    const T *z = static_cast<const T *>(dim == 3 ? d_z : d_y);
+    if (n <= kSmallPoints) {
+      small_kernel<<<1, 1024, 0, st>>>(x, y, z, n, dim, (T)rel, ctl);
+      return true;
+    }
+    if (cudaMemsetAsync(d_scratch, 0, kCtlBytes, st) != cudaSuccess) return false;
+    // enough blocks for the loads in flight, no more than the work fills
+    const uint64_t per_block = 256ull * kFoldUnroll * (16 / sizeof(T));
+    const int grid = (int)std::min<uint64_t>((uint64_t)num_sms() * 6, (n + per_block - 1) / per_block);
+    kernel<<<grid, 256, 0, st>>>(x, y, z, n, dim, (T)rel, ctl);
+    return true;
+  };
+  if (!(float_bits == 32 ? run(float(), rel_to_abs_small_kernel<float>, rel_to_abs_kernel<float>)
+                         : run(double(), rel_to_abs_small_kernel<double>, rel_to_abs_kernel<double>)))
+    return GPZ_ECUDA;
   if (cudaGetLastError() != cudaSuccess) return GPZ_ECUDA;
   Control h;
   if (cudaMemcpyAsync(&h, d_scratch, sizeof(Control), cudaMemcpyDeviceToHost, st) != cudaSuccess) return GPZ_ECUDA;

@@ -332,6 +332,28 @@ __global__ void __launch_bounds__(256, 6) strict_bound_kernel(const T *__restric
   }
 }
 
+// The segment-size rules on the sampled accumulators ([min inverted, max] per
+// axis) and their outcome in the control block (one thread).
+template <typename T>
+__device__ __forceinline__ void store_decision(const typename TT<T>::U (&acc)[6], uint32_t dim, uint32_t seg_in,
+                                               int rel_mode, T rel_eb, T ebv, int safe31, Control *ctl,
+                                               uint32_t *seg_out) {
+  using U = typename TT<T>::U;
+  T mm[6];
+#pragma unroll
+  for (uint32_t d = 0; d < 3; ++d) {
+    mm[d] = d < dim ? from_ord((U)~acc[2 * d]) : (T)0;
+    mm[3 + d] = d < dim ? from_ord(acc[2 * d + 1]) : (T)0;
+  }
+  const SegDecision sd = decide_seg<T>(mm, dim, seg_in, rel_mode, rel_eb, ebv, safe31);
+  if (seg_out) *seg_out = sd.status == kOK ? sd.seg : 0u;
+  if (sd.status != kOK) set_status(ctl, sd.status);
+  else {
+    ctl->seg = sd.seg;
+    ctl->adjusted = sd.adjusted;
+  }
+}
+
 // sampleMinMaxXYZKernel[2D] + reduceMinMax[2D] (src/cudaWarpCompress.cu:1216-1418):
 // 1024 windows of 256 consecutive points at stride max((N-256)/1024, 1).
 // A window that would run past N is skipped by the reference and its
@@ -389,26 +411,10 @@ __device__ __forceinline__ void seg_sample_block(const T *__restrict__ x, const 
   __syncthreads();
   if (last && threadIdx.x == 0) {
     __threadfence();
-    T mm[6];
-    for (uint32_t d = 0; d < 3; ++d) {
-      if (d < dim) {
-        const U mi = (U)(~(U)((volatile unsigned long long *)ctl->mm)[2 * d]);
-        const U ma = (U)((volatile unsigned long long *)ctl->mm)[2 * d + 1];
-        mm[d] = from_ord(mi);
-        mm[3 + d] = from_ord(ma);
-      } else {
-        mm[d] = 0;
-        mm[3 + d] = 0;
-      }
-    }
+    U all[6];
+    for (uint32_t k = 0; k < 6; ++k) all[k] = (U)((volatile unsigned long long *)ctl->mm)[k];
     const T ebv = eb_dev ? (T)*(const volatile double *)eb_dev : eb;
-    const SegDecision sd = decide_seg<T>(mm, dim, seg_in, rel_mode, rel_eb, ebv, safe31);
-    if (seg_out) *seg_out = sd.status == kOK ? sd.seg : 0u;
-    if (sd.status != kOK) set_status(ctl, sd.status);
-    else {
-      ctl->seg = sd.seg;
-      ctl->adjusted = sd.adjusted;
-    }
+    store_decision<T>(all, dim, seg_in, rel_mode, rel_eb, ebv, safe31, ctl, seg_out);
   }
 }
 
@@ -419,6 +425,66 @@ __global__ void __launch_bounds__(256) seg_sample_kernel(const T *__restrict__ x
                                                          int safe31, Control *ctl, const double *eb_dev) {
   if (eb_dev && ld_volatile(reinterpret_cast<const uint32_t *>(&ctl->status)) != 0) return;
   seg_sample_block<T>(x, y, z, n, dim, seg_in, rel_mode, rel_eb, eb, safe31, ctl, blockIdx.x, gridDim.x, eb_dev);
+}
+
+// Per-axis accumulators of a 1024-thread block's values, in every thread of the
+// first warp (lane k: accumulator k).
+template <typename U>
+__device__ __forceinline__ U block_max6(const U (&acc)[6], U (*red)[32]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const U v = warp_max(acc[k]);
+    if (lane == 0) red[k][warp] = v;
+  }
+  __syncthreads();
+  U mine = 0;
+  if (warp == 0) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const U v = warp_max(red[k][lane]);
+      if (lane == k) mine = v;
+    }
+  }
+  return mine;
+}
+
+// Snapshots of up to this many points take one block for what surrounds the
+// compress kernel (their look-back records all lie in the control block): the
+// clearing memset, the cross-block atomics and the last-block election go.
+constexpr uint64_t kSmallPoints = 16384;
+
+// seg_sample_kernel of a small snapshot, in one block that clears the control
+// block first.  Its windows overlap (stride <= 15), so they are one span of
+// the array, read once.  5,003 float points: 81 -> 77 us for the whole call
+// (with rel_to_abs_small_kernel) against a memset and 128 blocks.
+template <typename T>
+__global__ void __launch_bounds__(1024) seg_small_kernel(const T *__restrict__ x, const T *__restrict__ y,
+                                                         const T *__restrict__ z, uint64_t n, uint32_t dim,
+                                                         uint32_t seg_in, int rel_mode, T rel_eb, T eb, int safe31,
+                                                         Control *ctl) {
+  using U = typename TT<T>::U;
+  __shared__ U red[6][32];
+  if (threadIdx.x < kCtlBytes / 4) reinterpret_cast<uint32_t *>(ctl)[threadIdx.x] = 0u;
+  const uint64_t L = 256, B = 1024;
+  // windows inside the array, and the end of the last of them
+  const uint64_t stride = n >= L ? max((n - L) / B, (uint64_t)1) : 1, inside = n >= L ? min(B, (n - L) / stride + 1) : 0;
+  const uint64_t end = inside ? (inside - 1) * stride + L : 0;
+  U acc[6] = {0, 0, 0, 0, 0, 0};
+  if (inside < B) {  // the others contribute 0
+#pragma unroll
+    for (int d = 0; d < 3; ++d) fold_minmax<T>((T)0, acc[2 * d], acc[2 * d + 1]);
+  }
+  fold_axis<T>(x, end, 0, 1, acc[0], acc[1]);
+  fold_axis<T>(y, end, 0, 1, acc[2], acc[3]);
+  if (dim == 3) fold_axis<T>(z, end, 0, 1, acc[4], acc[5]);
+  const U mine = block_max6(acc, red);  // its barrier also orders the clearing before the result
+  if (threadIdx.x < 32) {
+    U all[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) all[k] = __shfl_sync(0xFFFFFFFFu, mine, k);
+    if (threadIdx.x == 0) store_decision<T>(all, dim, seg_in, rel_mode, rel_eb, eb, safe31, ctl, nullptr);
+  }
 }
 
 // The sampling windows of computeSegSize restricted to one shard
@@ -467,6 +533,33 @@ static __global__ void set_seg_kernel(Control *ctl, uint32_t seg) {
   ctl->adjusted = 0;
 }
 
+// The bound and the min / max from the accumulators ([min inverted, max] per
+// axis), one thread.
+template <typename T>
+__device__ __forceinline__ void store_rel_bound(const typename TT<T>::U (&acc)[6], T rel, Control *ctl, T *eb_out) {
+  using U = typename TT<T>::U;
+  T mn[3], mx[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    mn[d] = from_ord((U)~acc[2 * d]);
+    mx[d] = from_ord(acc[2 * d + 1]);
+    ctl->out_mm[d] = (double)mn[d];
+    ctl->out_mm[3 + d] = (double)mx[d];
+  }
+  T r;
+  if (sizeof(T) == 4) {
+    const float xr = __fsub_rn((float)mx[0], (float)mn[0]), yr = __fsub_rn((float)mx[1], (float)mn[1]);
+    const float zr = __fsub_rn((float)mx[2], (float)mn[2]);
+    r = (T)__fmul_rn(fmaxf(fmaxf(xr, yr), zr), (float)rel);
+  } else {
+    const double xr = __dsub_rn((double)mx[0], (double)mn[0]), yr = __dsub_rn((double)mx[1], (double)mn[1]);
+    const double zr = __dsub_rn((double)mx[2], (double)mn[2]);
+    r = (T)__dmul_rn(fmax(fmax(xr, yr), zr), (double)rel);
+  }
+  ctl->out_eb = (double)r;
+  if (eb_out) *eb_out = r;
+}
+
 // findMinimumValues<T> + convertRelEb<T> on the device.  The host scan starts
 // from float limits (include/utils.cuh:48-53) and ignores NaNs; 2D data has
 // z == 0 (utils.cuh:141).
@@ -508,25 +601,9 @@ __device__ __forceinline__ void rel_to_abs_block(const T *__restrict__ x, const 
   __syncthreads();
   if (last && threadIdx.x == 0) {
     __threadfence();
-    T mn[3], mx[3];
-    for (int d = 0; d < 3; ++d) {
-      mn[d] = from_ord((U)~(U)((volatile unsigned long long *)ctl->mm)[2 * d]);
-      mx[d] = from_ord((U)((volatile unsigned long long *)ctl->mm)[2 * d + 1]);
-      ctl->out_mm[d] = (double)mn[d];
-      ctl->out_mm[3 + d] = (double)mx[d];
-    }
-    T r;
-    if (sizeof(T) == 4) {
-      const float xr = __fsub_rn((float)mx[0], (float)mn[0]), yr = __fsub_rn((float)mx[1], (float)mn[1]);
-      const float zr = __fsub_rn((float)mx[2], (float)mn[2]);
-      r = (T)__fmul_rn(fmaxf(fmaxf(xr, yr), zr), (float)rel);
-    } else {
-      const double xr = __dsub_rn((double)mx[0], (double)mn[0]), yr = __dsub_rn((double)mx[1], (double)mn[1]);
-      const double zr = __dsub_rn((double)mx[2], (double)mn[2]);
-      r = (T)__dmul_rn(fmax(fmax(xr, yr), zr), (double)rel);
-    }
-    ctl->out_eb = (double)r;
-    if (eb_out) *eb_out = r;
+    U all[6];
+    for (int k = 0; k < 6; ++k) all[k] = (U)((volatile unsigned long long *)ctl->mm)[k];
+    store_rel_bound<T>(all, rel, ctl, eb_out);
   }
 }
 
@@ -535,6 +612,32 @@ __global__ void __launch_bounds__(256, 6) rel_to_abs_kernel(const T *__restrict_
                                                          const T *__restrict__ z, uint64_t n, uint32_t dim,
                                                          T rel, Control *ctl) {
   rel_to_abs_block<T>(x, y, z, n, dim, rel, ctl, nullptr, blockIdx.x, gridDim.x);
+}
+
+// The same for a small snapshot (kSmallPoints), in one block, without a cleared
+// control block.
+template <typename T>
+__global__ void __launch_bounds__(1024) rel_to_abs_small_kernel(const T *__restrict__ x, const T *__restrict__ y,
+                                                                const T *__restrict__ z, uint64_t n, uint32_t dim,
+                                                                T rel, Control *ctl) {
+  using U = typename TT<T>::U;
+  __shared__ U red[6][32];
+  U acc[6];
+  for (int d = 0; d < 3; ++d) {
+    acc[2 * d] = (U)~ord_of((T)FLT_MAX);
+    acc[2 * d + 1] = ord_of((T)(-FLT_MAX));
+  }
+  fold_axis<T>(x, n, 0, 1, acc[0], acc[1]);
+  fold_axis<T>(y, n, 0, 1, acc[2], acc[3]);
+  if (dim == 3) fold_axis<T>(z, n, 0, 1, acc[4], acc[5]);
+  else fold_minmax<T>((T)0, acc[4], acc[5]);
+  const U mine = block_max6(acc, red);
+  if (threadIdx.x < 32) {
+    U all[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) all[k] = __shfl_sync(0xFFFFFFFFu, mine, k);
+    if (threadIdx.x == 0) store_rel_bound<T>(all, rel, ctl, nullptr);
+  }
 }
 
 // ===========================================================================

@@ -73,3 +73,32 @@ def test_misaligned_axes(bits, shift):
     dt = np.float32 if bits == 32 else np.float64
     rng = np.random.default_rng(shift)
     check([(rng.random(40 * 1024 + 5) * 100).astype(dt) for _ in range(3)], 0.05, 4, shift)
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 1279, 1280, 1281, 2303, 2304, 5003, 16383, 16384, 16385])
+@pytest.mark.parametrize("rel", [1e-2, 1e-4])
+def test_automatic_segment_size_of_small_snapshots(bits, dim, n, rel):
+    """The one-block sampling (up to 16,384 points, scratch not cleared) against the oracle's windows."""
+    dt = np.float32 if bits == 32 else np.float64
+    rng = np.random.default_rng(n + dim)
+    axes = [(5.0 + 10.0 ** d * rng.random(n)).astype(dt) for d in range(dim)]
+    axes[0][-1] = 400.0  # outside the last window of many sizes
+    z = axes[2] if dim == 3 else np.zeros_like(axes[0])
+    relT = float(dt(rel))
+    eb = po.rel_to_abs(axes[0], axes[1], z if dim == 3 else None, relT)
+    dev = [torch.from_numpy(a).cuda() for a in axes]
+    got_eb, _ = gz.rel_to_abs(dev[0], dev[1], dev[2] if dim == 3 else None, relT)
+    assert got_eb == eb
+    if eb == 0.0:  # one point in 3D: no range, no bound to compress with
+        return
+    seg, _ = po.seg_size(axes[0], axes[1], z, dim, 0, True, relT, eb)
+    want = po.compress(axes[0], axes[1], z, dim, eb, seg)
+    out = torch.zeros(gz.stream_bound(n, dim, bits), dtype=torch.uint8, device="cuda")
+    scratch = torch.full((gz.compress_scratch_bytes(n),), 255, dtype=torch.uint8, device="cuda")
+    p = gz.make_params(n, dim, bits, eb, rel_mode=True, rel_eb=relT)
+    for _ in range(2):
+        r = gz.compress_into(p, dev[0], dev[1], dev[2] if dim == 3 else dev[0], out, scratch)
+        assert (r.status, r.seg_size) == (0, seg)
+        assert out[: r.stream_bytes].cpu().numpy().tobytes() == want
