@@ -4,7 +4,7 @@
 // The reference compresses one snapshot per call (CompressorManager::compressWarp,
 // src/CompressorManager.cpp:12-16), so a workload of many small snapshots is
 // dominated by per-call launches, syncs and an almost idle GPU.  Here every
-// snapshot keeps its own stream, control block and look-back words; the
+// snapshot keeps its own stream, control block and look-back records; the
 // chunks of all snapshots of a class form one global work list (snapshot
 // after snapshot, so each snapshot's chunks are claimed in order), and one
 // persistent kernel per class claims them.  A snapshot's stream is

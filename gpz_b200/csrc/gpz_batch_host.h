@@ -2,7 +2,7 @@
 // plans (gpz_batchapi.cu) and the request server (gpz_serve.cu).
 //
 // A batch runs in a workspace of device memory laid out by *_layout:
-//   [0, zero_bytes)      control blocks, look-back words, work counters;
+//   [0, zero_bytes)      control blocks, look-back records, work counters;
 //                        cleared by *_enqueue before the kernels run
 //   [zero_bytes, bytes)  descriptors and work maps, built on the host by
 //                        *_tables into a host image of that range
@@ -32,7 +32,7 @@ struct ClassPlan {
 
 struct Layout {
   ClassPlan cls[4];                // (float, 2D), (float, 3D), (double, 2D), (double, 3D)
-  std::vector<uint64_t> look_off;  // compress: each item's look-back words
+  std::vector<uint64_t> look_off;  // compress: each item's look-back records after the first
   uint64_t claim_off = 0, zero_bytes = 0, bytes = 0;
   uint32_t count = 0;
 };

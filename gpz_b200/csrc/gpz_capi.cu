@@ -503,8 +503,8 @@ int gpz_stream_size(const void *d_stream, uint64_t cap, uint64_t *bytes, void *s
 // by an application that owns the whole device-memory budget and only hands
 // out the input and output buffers, or a latency-critical path where the
 // implicit device synchronisation of cudaMalloc is not acceptable.  For them
-// gpz_compress_noalloc takes its scratch (control block + one look-back word
-// per 1024-point chunk) from a fixed array compiled into this library instead
+// gpz_compress_noalloc takes its scratch (control block + look-back
+// records) from a fixed array compiled into this library instead
 // of from the caller.
 // ===========================================================================
 namespace {
@@ -549,7 +549,7 @@ int gpz_compress_noalloc(const gpz_params *params, const void *d_x, const void *
   void *scratch = nullptr;
   int rc = noalloc_scratch(&scratch);
   if (rc) return rc;
-  // gpz_compress_async clears the control block and the look-back words it
+  // gpz_compress_async clears the control block and the look-back records it
   // uses, so the previous call's leftovers in the shared array do not matter.
   rc = gpz_compress_async(params, d_x, d_y, d_z, d_out, out_capacity, scratch, kNoAllocScratchBytes, stream);
   if (rc) return rc;
@@ -560,7 +560,7 @@ int gpz_compress_noalloc(const gpz_params *params, const void *d_x, const void *
 
 // ---------------------------------------------------------------------------
 // Check of the bounded wait of the placement look-back: group 1 waits on a
-// group 0 that never publishes its size (its look-back word stays zero, as if
+// group 0 that never publishes its size (its field of the record stays zero, as if
 // the CTA holding it had stopped), so the wait runs out after `polls` polls.
 // ---------------------------------------------------------------------------
 namespace {

@@ -98,7 +98,7 @@ typedef struct gpz_result {
 uint64_t gpz_stream_bound(uint64_t n, uint32_t dim, uint32_t float_bits);
 
 /* Device scratch needed by gpz_compress_async for n points (control block
- * plus one 8-byte look-back word per 1024-point chunk).  Replaces the
+ * plus 8 bytes per 1024-point chunk for the look-back records).  Replaces the
  * caller-provided 4*N*sizeof(T) scratch of ICudaCompressor::compress
  * (reference include/ICudaCompressor.cuh:10-11, src/main.cpp:289-291). */
 uint64_t gpz_compress_scratch_bytes(uint64_t n);
@@ -268,13 +268,13 @@ int gpz_stream_size(const void *d_stream, uint64_t cap, uint64_t *bytes, void *s
  * samples, launches and synchronises on its own).  A batch compresses many
  * snapshots of mixed size, float width and dimension with one CUDA graph:
  * device rel->abs bounds, segment-size sampling and one persistent compress
- * kernel per (float width, dimension) class whose work list holds the 8-chunk
- * groups of all its snapshots.  Every snapshot's stream is byte-identical to
+ * kernel per (float width, dimension) class whose work list holds the chunks
+ * of all its snapshots.  Every snapshot's stream is byte-identical to
  * what gpz_compress writes for the same parameters.
  *
  * A batch is a plan bound to the buffers named in its items (like an FFT
  * plan): gpz_batch_create validates the items, allocates the batch's device
- * memory (descriptors, work maps, one control block and look-back words per
+ * memory (descriptors, work maps, control blocks and look-back records per
  * snapshot) and captures the graph; gpz_batch_launch replays it on a stream
  * (the inputs may change between launches, the pointers and sizes may not);
  * gpz_batch_results synchronises the stream and reads every snapshot's result.
