@@ -722,7 +722,7 @@ def run_batched(args):
 
     nb_snap = [x.numel() * (3 if z is not None else 2) * (4 if x.dtype == torch.float32 else 8)
                for x, _, z, _ in snaps]
-    wave_chunks = 2 * 148 * 8  # resident CTAs x SMs x chunks per CTA on a B200
+    wave_chunks = 6 * 148  # resident compress CTAs (one chunk each) x SMs on a B200
     large = [x.numel() >= wave_chunks * 1024 for x, _, _, _ in snaps]
     c_calls = [(lambda x=x, y=y, z=z, p=p, o=o, sc=sc: gz.compress_into(p, x, y, z if z is not None else x, o, sc,
                                                                          stream, sync=False))
@@ -802,8 +802,8 @@ def run_batched(args):
                       "segments_changed": sum(a != b for a, b in zip(segs_default, segs_tuned)),
                       "candidates": [1, 2, 4, 8, 16, 32, 64, 128], "sample_points": 1 << 17},
         "identical_output": bool(same),
-        "ceiling": {"note": "snapshots of at least one wave of the persistent compress grid (2 CTAs x 148 SMs x 8 "
-                            "chunks = 2,424,832 points) keep the GPU busy alone; the best a batch can do is run "
+        "ceiling": {"note": "snapshots of at least one wave of the persistent compress grid (6 CTAs x 148 SMs, one "
+                            "chunk each = 909,312 points) keep the GPU busy alone; the best a batch can do is run "
                             "the smaller ones at the large ones' rate",
                     "wave_points": wave_chunks * 1024, "compress": ceil_c, "decompress": ceil_d},
     }

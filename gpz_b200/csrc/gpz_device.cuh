@@ -111,7 +111,6 @@ __host__ __device__ __forceinline__ double from_ord(unsigned long long o) {
 
 // Warp-wide max of 32/64-bit unsigned values (REDUX on sm_80+).
 __device__ __forceinline__ uint32_t warp_max(uint32_t v) { return __reduce_max_sync(0xFFFFFFFFu, v); }
-__device__ __forceinline__ uint32_t warp_min(uint32_t v) { return __reduce_min_sync(0xFFFFFFFFu, v); }
 __device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
   uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)(v >> 32));
   uint32_t lo = __reduce_max_sync(0xFFFFFFFFu, ((uint32_t)(v >> 32) == hi) ? (uint32_t)v : 0u);
@@ -210,24 +209,6 @@ __host__ __device__ __forceinline__ int swz(int i) { return i ^ ((i >> 3) & 0x1C
 // touching the same quad of their rows (or 8 quads of one row) hit 8
 // different bank groups.
 __device__ __forceinline__ uint32_t qoff(int row, int m) { return 32u * row + ((uint32_t)((m ^ row) & 7) << 2); }
-
-// Loads the 32 values of group g (elements 32g..32g+31) from a swizzled array.
-__device__ __forceinline__ void load_group(const uint32_t *arr, int g, uint32_t (&a)[32]) {
-  const uint4 *p = reinterpret_cast<const uint4 *>(arr + 32 * g);
-#pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const uint4 v = p[m ^ (g & 7)];
-    a[4 * m + 0] = v.x;
-    a[4 * m + 1] = v.y;
-    a[4 * m + 2] = v.z;
-    a[4 * m + 3] = v.w;
-  }
-}
-__device__ __forceinline__ void store_group(uint32_t *arr, int g, const uint32_t (&a)[32]) {
-  uint4 *p = reinterpret_cast<uint4 *>(arr + 32 * g);
-#pragma unroll
-  for (int m = 0; m < 8; ++m) p[m ^ (g & 7)] = make_uint4(a[4 * m], a[4 * m + 1], a[4 * m + 2], a[4 * m + 3]);
-}
 
 // ---------------------------------------------------------------------------
 // In-register 32x32 bit transposes.  Input a[k] = value of element k; output

@@ -60,7 +60,8 @@ static_assert(kEncSlots >= 2, "the oldest payload is looked up while the newest 
 static_assert(kChunk / kEncWarps + 2 * kEncHalo == 32 * kEncOrd, "ordering window");
 static_assert(kEncHalo >= kEncSmall - 1, "a small bucket must fit the halo");
 
-// Batcher's odd-even merge sort network on 32 values (191 exchanges).
+// Batcher's odd-even merge sort network on 32 values (191 exchanges).  No kernel
+// sorts with it any more; its CPU check (tests/host/network_check.cu) stays.
 __host__ __device__ __forceinline__ void oem_sort32(uint32_t (&a)[32]) {
 #pragma unroll
   for (int p = 1; p < 32; p <<= 1)
