@@ -402,16 +402,15 @@ struct FastDiv31 {
   }
 };
 
-// Relaxed GPU-scope accesses for the look-back records.
+// Relaxed GPU-scope accesses for the look-back records.  A vector access is one
+// access per element, in no order: the loads' elements are 64 bits wide like the
+// words that the ORs set, so that every word is read as it stood at one time.
 __device__ __forceinline__ void red_or_relaxed(unsigned long long *p, unsigned long long v) {
   asm volatile("red.relaxed.gpu.global.or.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ uint4 ld_relaxed4(const uint4 *p) {
-  uint4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p)
-               : "memory");
+__device__ __forceinline__ ulonglong2 ld_relaxed2(const unsigned long long *p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p) { return *(const volatile uint32_t *)p; }

@@ -662,9 +662,12 @@ struct CArgs {
 // (five to a word, the sixteenth on top of the last word; zero until it is
 // known), and below that the group's prefix -- the stream offset of its first
 // chunk in 4-byte units -- with kLookKnown once somebody has it.  Every field
-// is set by one relaxed atomic OR and valid by itself, so neither side needs
-// a fence (an offset kept beside its flag cost two per chunk, 4-5 thousand
-// cycles under load).
+// lies in one word, is set by one relaxed atomic OR of that word and read with
+// the whole word, so it is valid by itself and neither side needs a fence (an
+// offset kept beside its flag cost two per chunk, 4-5 thousand cycles under
+// load).  The two 16-byte loads a record takes have 64-bit elements: with
+// 32-bit ones the sizes of every third chunk and the prefix span two elements,
+// which nothing orders.
 //
 // A chunk's offset is the nearest known prefix at or below its own group plus
 // the sizes from there on; a step reads 512 predecessors, one record a lane,
@@ -688,12 +691,20 @@ __device__ __forceinline__ unsigned long long *look_record(Control *ctl, unsigne
   return g == 0 ? reinterpret_cast<unsigned long long *>(reinterpret_cast<uint8_t *>(ctl) + kLookTail) : look + 4 * g;
 }
 
+// The word and the lowest bit of the size of a record's chunk i.
+__host__ __device__ constexpr uint32_t look_word(uint32_t i) { return i == 15u ? 3u : i / 5u; }
+__host__ __device__ constexpr uint32_t look_shift(uint32_t i) { return i == 15u ? 52u : 12u * (i % 5u); }
+
+// Size of a record's chunk i (4-byte units; 0: not known yet) in its words.
+__host__ __device__ __forceinline__ uint32_t look_size(const unsigned long long (&w)[4], uint32_t i) {
+  return (uint32_t)(w[look_word(i)] >> look_shift(i)) & 4095u;
+}
+
 // One thread: the payload size of chunk c (bytes, a multiple of 4, not 0).
 __device__ __forceinline__ void publish_size(Control *ctl, unsigned long long *look, unsigned long long c,
                                              uint32_t bytes) {
-  const uint32_t i = (uint32_t)c & (kLookGroup - 1u), w = i / 5u;  // chunk 15: word 3
-  const uint32_t sh = i == 15u ? 52u : 12u * (i - 5u * w);
-  red_or_relaxed(look_record(ctl, look, c / kLookGroup) + w, (unsigned long long)(bytes >> 2) << sh);
+  const uint32_t i = (uint32_t)c & (kLookGroup - 1u);
+  red_or_relaxed(look_record(ctl, look, c / kLookGroup) + look_word(i), (unsigned long long)(bytes >> 2) << look_shift(i));
 }
 
 // Warp-collective: the stream offset of chunk c, and its group's prefix for
@@ -712,25 +723,22 @@ static __device__ int resolve_prefix(Control *ctl, unsigned long long *look, uns
   uint32_t spins = 0, backoff = 32;
   for (;;) {
     const long long g = top - 31 + lane;
-    uint4 q0 = make_uint4(0u, 0u, 0u, 0u), q1 = q0;
+    ulonglong2 q0 = make_ulonglong2(0ull, 0ull), q1 = q0;
     if (g >= 0) {
-      const uint4 *const rec = reinterpret_cast<const uint4 *>(look_record(ctl, look, (unsigned long long)g));
-      q0 = ld_relaxed4(rec);
-      q1 = ld_relaxed4(rec + 1);
+      const unsigned long long *const rec = look_record(ctl, look, (unsigned long long)g);
+      q0 = ld_relaxed2(rec);
+      q1 = ld_relaxed2(rec + 2);
     }
-    const unsigned long long w3 = ((unsigned long long)q1.w << 32) | q1.z;
-    const bool known = g <= 0 || (w3 & kLookKnown) != 0ull;
+    const unsigned long long w[4] = {q0.x, q0.y, q1.x, q1.y};
+    const bool known = g <= 0 || (w[3] & kLookKnown) != 0ull;
     const int near = 31 - __clz((int)__ballot_sync(FULL, known));  // -1: none in the window
     // sizes of this lane's chunks before c
     const uint32_t cnt = g == (long long)(c / kLookGroup) ? own : (uint32_t)kLookGroup;
-    const uint32_t lo[3] = {q0.x, q0.z, q1.x}, hi[3] = {q0.y, q0.w, q1.y};
     uint32_t sum = 0;
     bool missing = false;
 #pragma unroll
     for (uint32_t i = 0; i < (uint32_t)kLookGroup; ++i) {
-      const uint32_t w = i < 15u ? i / 5u : 2u, sh = 12u * (i % 5u);
-      const uint32_t v = i == 15u ? q1.w >> 20
-                                  : (sh >= 32u ? hi[w] >> (sh - 32u) : __funnelshift_r(lo[w], hi[w], sh)) & 4095u;
+      const uint32_t v = look_size(w, i);
       if (i < cnt) {
         sum += v;
         missing |= v == 0u;
@@ -753,7 +761,7 @@ static __device__ int resolve_prefix(Control *ctl, unsigned long long *look, uns
     excl += __reduce_add_sync(FULL, counts ? sum : 0u);
     if (top == (long long)(c / kLookGroup)) in_group = __shfl_sync(FULL, sum, 31);
     if (near >= 0) {
-      const unsigned long long pre = g <= 0 ? 0ull : (w3 & kLookPrefix);
+      const unsigned long long pre = g <= 0 ? 0ull : (w[3] & kLookPrefix);
       excl += __shfl_sync(FULL, pre, near);
       // the group's prefix, unless it is there (setting it again changes nothing)
       if (lane == 31 && !(top == (long long)(c / kLookGroup) && near == 31))
