@@ -15,8 +15,9 @@
 //      out the chunk's scalars;
 //   2. rank: 1024 buckets over the id range (shared-atomic counts, scan,
 //      placement at bucket start + arrival slot, then odd-even transposition
-//      between neighbouring positions); a chunk with few distinct ids or a
-//      crowded bucket goes through a stable radix sort instead;
+//      between neighbouring positions); a chunk with too crowded a bucket goes
+//      through a comparison network of the whole CTA (ids below 2^22) or a
+//      stable radix sort (wider ids, and the few ids of one radix pass);
 //   3. runs of equal ids (unique ids, deltas, counts), the payload's size,
 //      which is published at once for the chunks behind;
 //   4. bit planes, eight at a time per warp, into a staged payload, which
@@ -47,7 +48,8 @@ constexpr int kEncThreads = 128;          // threads (one chunk) per CTA
 constexpr int kEncWarps = kEncThreads / 32;
 constexpr int kEncPer = kChunk / kEncThreads;  // points per thread
 constexpr int kEncBuckets = 1024;         // ranking buckets per chunk
-constexpr int kEncBucketBits = 11;        // id ranges below 2^11 skip the buckets
+constexpr int kEncBucketBits = 11;        // no kernel uses it any more; a CPU check (tests/host/bucket_check.cu) does
+constexpr uint32_t kEncOnePass = 512;     // ids below this: one radix pass, no buckets
 constexpr int kEncSmall = 16;             // a bucket of this many points or more is sorted on its own
 constexpr int kEncCrowd = 256;            // one above this size declines the chunk, and so do more than
 constexpr int kEncCrowdPoints = 512;      //   this many points in all buckets of kEncSmall or more
@@ -214,8 +216,8 @@ __device__ __forceinline__ uint32_t warp_inc_scan(uint32_t v, int lane) {
   return v;
 }
 
-// Stable radix sort of the chunk by block id, for chunks the buckets do not
-// suit (few distinct ids, a crowded bucket, a short last chunk): least
+// Stable radix sort of the chunk by block id, for chunks of up to kEncOnePass
+// ids, of wide ids with too crowded a bucket, and a short last chunk: least
 // significant digit first over the points in rank order, so equal ids keep
 // the order of their ranks.  A warp takes 256 consecutive elements, 32 at a
 // time; lanes of one digit find each other by match.any and the first of them
@@ -287,52 +289,52 @@ static __device__ __noinline__ const uint16_t *radix_rank(const uint32_t *byr, u
   return perm + ((passes + 1u) & 1u) * kChunk;
 }
 
-// Ascending sort of the n <= 32 K distinct values a[0..n) by one warp, K a
-// lane (lane l: values K l ..): a bitonic network whose exchanges all put the
-// minimum at the lower index (the first step of each merge pairs i with
-// i ^ (k - 1)), padded with the largest value.  Partners in other lanes come
-// by shuffles: about 60 / 150 / 250 / 460 instructions for K = 1 / 2 / 4 / 8,
-// where the same network in shared memory took 2,000 for 256 values.
+// Compare-exchange step j of a bitonic merge of k values (lane l: positions
+// K l ..): the merge's first step (j = k / 2) pairs position i with i ^ (k - 1),
+// the others i with i ^ j, so the minimum always goes to the lower position.
+// Partners in other lanes come by shuffles.
 template <int K>
-__device__ __forceinline__ void warp_sort_regs(uint32_t *a, uint32_t n, int lane) {
-  constexpr uint32_t FULL = 0xFFFFFFFFu;
-  uint32_t v[K];
+__device__ __forceinline__ void exchange(uint32_t (&v)[K], int lane, int k, int j) {
+  const bool mirror = j == (k >> 1);
+  if (j < K) {  // both in this lane
 #pragma unroll
-  for (int e = 0; e < K; ++e) v[e] = (uint32_t)(K * lane + e) < n ? a[K * lane + e] : FULL;
-#pragma unroll
-  for (int k = 2; k <= 32 * K; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      const bool mirror = j == (k >> 1);
-      if (j < K && k <= K) {  // both in this lane
-#pragma unroll
-        for (int e = 0; e < K; ++e) {
-          const int p = mirror ? e ^ (k - 1) : e ^ j;
-          if (e < p) {
-            const uint32_t x = v[e], y = v[p];
-            v[e] = min(x, y);
-            v[p] = max(x, y);
-          }
-        }
-      } else if (j < K) {  // past a merge's first step, inside the lane
-#pragma unroll
-        for (int e = 0; e < K; ++e)
-          if ((e & j) == 0) {
-            const uint32_t x = v[e], y = v[e | j];
-            v[e] = min(x, y);
-            v[e | j] = max(x, y);
-          }
-      } else {
-        const int m = mirror ? k / K - 1 : j / K;  // partner lane ^ m
-        const bool upper = (lane & (j / K)) != 0;
-        uint32_t o[K];
-#pragma unroll
-        for (int e = 0; e < K; ++e) o[e] = __shfl_xor_sync(FULL, v[mirror ? K - 1 - e : e], m);
-#pragma unroll
-        for (int e = 0; e < K; ++e) v[e] = upper ? max(v[e], o[e]) : min(v[e], o[e]);
+    for (int e = 0; e < K; ++e) {
+      const int p = mirror ? e ^ (k - 1) : e ^ j;
+      if (e < p) {
+        const uint32_t x = v[e], y = v[p];
+        v[e] = min(x, y);
+        v[p] = max(x, y);
       }
     }
+  } else {
+    const int m = mirror ? k / K - 1 : j / K;  // partner lane ^ m
+    const bool upper = (lane & (j / K)) != 0;
+    uint32_t o[K];
+#pragma unroll
+    for (int e = 0; e < K; ++e) o[e] = __shfl_xor_sync(0xFFFFFFFFu, v[mirror ? K - 1 - e : e], m);
+#pragma unroll
+    for (int e = 0; e < K; ++e) v[e] = upper ? max(v[e], o[e]) : min(v[e], o[e]);
   }
+}
+
+// Ascending sort of a warp's 32 K values: about 60 / 150 / 250 / 460
+// instructions for K = 1 / 2 / 4 / 8, where the same network in shared memory
+// took 2,000 for 256 values.
+template <int K>
+__device__ __forceinline__ void warp_sort(uint32_t (&v)[K], int lane) {
+#pragma unroll
+  for (int k = 2; k <= 32 * K; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) exchange<K>(v, lane, k, j);
+}
+
+// The same of the n <= 32 K distinct values a[0..n), padded with the largest value.
+template <int K>
+__device__ __forceinline__ void warp_sort_regs(uint32_t *a, uint32_t n, int lane) {
+  uint32_t v[K];
+#pragma unroll
+  for (int e = 0; e < K; ++e) v[e] = (uint32_t)(K * lane + e) < n ? a[K * lane + e] : 0xFFFFFFFFu;
+  warp_sort<K>(v, lane);
 #pragma unroll
   for (int e = 0; e < K; ++e)
     if ((uint32_t)(K * lane + e) < n) a[K * lane + e] = v[e];
@@ -343,6 +345,57 @@ static __device__ __noinline__ void warp_sort_small(uint32_t *a, uint32_t n, int
   else if (n <= 64u) warp_sort_regs<2>(a, n, lane);
   else if (n <= 128u) warp_sort_regs<4>(a, n, lane);
   else warp_sort_regs<8>(a, n, lane);
+}
+
+// Sort of a full chunk's 1024 composites id << 10 | rank (ids below 2^22) by
+// the CTA, for chunks the buckets have declined: each warp sorts 256 in
+// registers; the two merges above that take three exchanges between warps,
+// through S and H in turn.  S: ids by rank (rx); H: the sorted composites.
+// Begins and ends with a barrier.
+//
+// Bound by instruction issue: 700 instructions a warp and five barriers, on any
+// input.  The radix sort takes 350 and six barriers a pass, and two or three
+// passes at these ids: 20M float points, half of them in one place, 396 -> 296
+// us in 2D (19-bit ids) and 419 -> 309 us in 3D (21 bits), 292 -> 280 us with
+// ids of two passes; 3D points on 40 sites 366 -> 296 us.
+static __device__ __noinline__ void cta_sort(uint32_t *H, uint32_t *S) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  uint32_t v[kEncPer];
+  auto get = [](const uint32_t *buf, int from, uint32_t (&o)[kEncPer]) {
+    const uint4 a = ld4(buf + 4 * from), b = ld4(buf + 4 * (kEncThreads + from));
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+    o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+  };
+  // position 8t + e against thread `from`'s e (mirror: 7 - e); the upper takes the larger
+  auto cross = [&](uint32_t *buf, int from, bool mirror, bool upper) {
+    *reinterpret_cast<uint4 *>(buf + 4 * t) = make_uint4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<uint4 *>(buf + 4 * (kEncThreads + t)) = make_uint4(v[4], v[5], v[6], v[7]);
+    __syncthreads();
+    uint32_t o[kEncPer];
+    get(buf, from, o);
+#pragma unroll
+    for (int e = 0; e < kEncPer; ++e) {
+      const uint32_t y = o[mirror ? kEncPer - 1 - e : e];
+      v[e] = upper ? max(v[e], y) : min(v[e], y);
+    }
+  };
+  auto finish = [&]() {  // within the warp's 256 positions
+#pragma unroll
+    for (int j = 16 * kEncPer; j > 0; j >>= 1) exchange<kEncPer>(v, lane, 0, j);
+  };
+  __syncthreads();  // the ids by rank are in place
+#pragma unroll
+  for (int e = 0; e < kEncPer; ++e) v[e] = (S[rx(kEncPer * t + e)] << 10) | (uint32_t)(kEncPer * t + e);
+  warp_sort<kEncPer>(v, lane);
+  cross(H, t ^ 63, true, (warp & 1) != 0);    // i with i ^ 511
+  finish();
+  cross(S, t ^ 127, true, (warp & 2) != 0);   // i with i ^ 1023
+  cross(H, t ^ 32, false, (warp & 1) != 0);   // i with i ^ 256
+  finish();
+  __syncthreads();  // H has been read
+  *reinterpret_cast<uint4 *>(H + 8 * t) = make_uint4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<uint4 *>(H + 8 * t + 4) = make_uint4(v[4], v[5], v[6], v[7]);
+  __syncthreads();
 }
 
 // A chunk's points in registers, one 16-byte load (kVec points) at a time:
@@ -365,7 +418,8 @@ struct Points {
 
 // Ranks a full chunk's points through buckets over their id range.
 //  * kNarrow (ids below 2^22): 1024 buckets that split the range evenly
-//    (id * scale >> 32); S holds whole composites id << 10 | r.  H receives
+//    (id * scale >> 32; up to 1023 ids each have their own, but for the first
+//    two); S holds whole composites id << 10 | r.  H receives
 //    the sorted composites.
 //  * wide: buckets are the id bits from `low` up; S holds the bits below with
 //    r, and the bucket of every position lies beside (in Q).  H receives the
@@ -386,7 +440,8 @@ __device__ __forceinline__ bool rank_buckets(RankShared &sm, uint32_t *H, uint32
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t rbase = Points<T>::rank_base(t);
   const uint32_t low = kNarrow ? 0u : 22u - __clz(bound);  // wide: id bits below the bucket
-  // 1024 * 2^32 / (bound + 1), a little less: id * scale >> 32 <= 1023
+  // 1024 * 2^32 / (bound + 1), a little less: id * scale >> 32 <= 1023 (at
+  // most 2^32 - 1, with which it is id - 1)
   const uint32_t scale = kNarrow ? __float2uint_rz(__fdividef(4.39804e12f, __uint2float_rn(bound) + 1.0f)) : 0u;
   uint32_t bs[kEncPer];  // arrival slot << 14 | bucket << 2
 #pragma unroll
@@ -605,9 +660,13 @@ __device__ __forceinline__ void prefetch_points(const CArgs<T> &a, unsigned long
   }
 }
 
-// Ranks a chunk's points by (block id, r): narrow buckets (1: H holds the
-// sorted composites), wide buckets (2: H the sorted ids, `ranks` the ranks) or
-// the radix sort (0: S the ids by rank, rx, `ranks` the ranks).  No id is above
+// Ranks a chunk's points by (block id, r): narrow buckets or the CTA's network
+// (1: H holds the sorted composites), wide buckets (2: H the sorted ids, `ranks`
+// the ranks) or the radix sort (0: S the ids by rank, rx, `ranks` the ranks).
+// Full chunks of more than kEncOnePass ids try the buckets: spread evenly over
+// 1,250 ids, 20M float 2D points took 313 us when ids below 2^11 went to two
+// radix passes, 193 us so; at 441 ids one radix pass takes 276, what the buckets
+// would gain there few inputs show.  No id is above
 // `bound`; positions past the end of a short chunk rank last.  rank_skip counts
 // the chunks still to sort without trying the buckets, declined the chunks the
 // buckets have declined in a row.
@@ -617,7 +676,7 @@ __device__ __forceinline__ int rank_chunk(RankShared &sm, uint32_t *H, uint32_t 
                                           int t, int lane, int warp, const uint16_t *&ranks) {
   const bool full = nvalid == (uint32_t)kChunk, narrow = bound < (1u << 22);
   int how = 0;
-  if (full && bound >= (1u << kEncBucketBits) && rank_skip == 0u) {
+  if (full && bound >= kEncOnePass && rank_skip == 0u) {
     if (narrow) how = rank_buckets<T, true>(sm, H, S, key, bound, t, lane, warp) ? 1 : 0;
     else how = rank_buckets<T, false>(sm, H, S, key, bound, t, lane, warp) ? 2 : 0;
     // one crowded chunk says little about the next (a shuffled, clustered
@@ -637,6 +696,10 @@ __device__ __forceinline__ int rank_chunk(RankShared &sm, uint32_t *H, uint32_t 
     }
 #pragma unroll
     for (int e = 0; e < kEncPer; ++e) S[rx(rbase + Points<T>::rank_step(e))] = key[e];
+    if (full && narrow && bound >= kEncOnePass) {
+      cta_sort(H, S);
+      return 1;
+    }
     ranks = radix_rank(S, H, reinterpret_cast<uint16_t *>(sm.Q), sm.tot, bitlen(bound + (full ? 0u : 1u)));
   }
   return how;
