@@ -2,7 +2,7 @@
 
 A `Batch` is a plan bound to its snapshots' device buffers: it is created
 once (validation, device memory for descriptors and per-snapshot control
-blocks, CUDA-graph capture) and launched any number of times; each launch
+blocks, the CUDA graph) and launched any number of times; each launch
 compresses every snapshot, and each snapshot's stream is byte-identical to
 what `gpz_b200.compress` writes with the same parameters.  The reference has
 no batched form (one snapshot per CompressorManager::compressWarp call,

@@ -6,9 +6,9 @@
 //                        cleared by *_enqueue before the kernels run
 //   [zero_bytes, bytes)  descriptors and work maps, built on the host by
 //                        *_tables into a host image of that range
-// *_enqueue clears the first range and launches the class kernels on a
-// stream; it allocates nothing, so it runs inside a graph capture (the batch
-// plans) or directly (the server, which uploads the table image itself).
+// *_enqueue clears the first range and launches the class kernels on a stream
+// (the server, which uploads the table image itself); a batch plan puts the
+// same launches in a graph.  Neither allocates device memory.
 #pragma once
 
 #include <cstdint>
@@ -50,11 +50,10 @@ bool decompress_layout(const gpz_dbatch_item *items, uint32_t count, Layout &L);
 void compress_tables(const gpz_batch_item *items, const Layout &L, uint8_t *dev, uint8_t *image);
 void decompress_tables(const gpz_dbatch_item *items, const Layout &L, uint8_t *dev, uint8_t *image);
 
-// Clears the control range and launches the class kernels on `st`: one class
-// after another, or, with `branches` on a capturing stream, as parallel
-// branches of the graph.
-void compress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st, bool branches = false);
-void decompress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st, bool branches = false);
+// Clears the control range and launches the class kernels on `st`, one class
+// after another.
+void compress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st);
+void decompress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st);
 
 // Item i's control block (compress: also its rel->abs block at count + i).
 inline uint64_t ctl_off(uint32_t i) { return (uint64_t)i * 256u; }

@@ -1,20 +1,21 @@
 // gpz_batchapi.cu -- batched compress / decompress: workspace layout, table
 // building and kernel launches (gpz_batch_host.h), and the plan API of
-// include/gpz_b200.h (gpz_batch_*, gpz_dbatch_*), which captures them in a
-// CUDA graph.
+// include/gpz_b200.h (gpz_batch_*, gpz_dbatch_*), which puts them in a CUDA
+// graph.
 //
 // Classes are (float, 2D), (float, 3D), (double, 2D), (double, 3D): (compress)
 // rel->abs when any of its snapshots asks for it, sampling, one persistent
 // compress kernel; (decompress) a header check per stream, one persistent
 // decompress kernel.  A plan's graph runs its classes as parallel branches, so
-// that a class's launches and last chunks overlap the others' work: 368 -> 294
-// us for 48 mixed snapshots of 10,000 to 1.2M points, 137 -> 64 us for 16 of
+// that a class's launches and last chunks overlap the others' work: 368 -> 290
+// us for 48 mixed snapshots of 10,000 to 1.2M points, 137 -> 57 us for 16 of
 // 1,600 to 200,000.  The server's batches run them one after another on the
 // slot's stream.
 
 #include <algorithm>
 #include <cstring>
 #include <new>
+#include <tuple>
 #include <vector>
 
 #include "gpz_b200.h"
@@ -102,68 +103,123 @@ int dec_grid(uint64_t chunks) {
   return o ? (int)std::min<uint64_t>((chunks + W - 1) / W, (uint64_t)current_sms() * o) : -1;
 }
 
-template <typename T, int DIM>
-void enqueue_class(const gpzb_host::ClassPlan &cp, uint32_t count, uint8_t *dev, uint64_t claim_off, cudaStream_t st) {
-  BItem<T> *tab = reinterpret_cast<BItem<T> *>(dev + cp.table_off);
-  if (cp.rel_blocks)
-    batch_rel_mapped_kernel<T><<<(unsigned)cp.rel_blocks, 256, 0, st>>>(
-        tab, reinterpret_cast<const unsigned long long *>(dev + cp.rmap_off), count);
-  batch_sample_kernel<T><<<dim3(128, (unsigned)cp.items.size()), 256, 0, st>>>(tab);
-  compress_batch_kernel<T, DIM><<<cp.grid, kEncThreads, sizeof(EncShared), st>>>(
-      tab, (uint32_t)cp.items.size(), cp.work, reinterpret_cast<unsigned long long *>(dev + claim_off));
-}
-
-template <typename T, int DIM>
-void enqueue_dclass(const gpzb_host::ClassPlan &cp, uint8_t *dev, cudaStream_t st) {
-  DItem<T> *tab = reinterpret_cast<DItem<T> *>(dev + cp.table_off);
-  const uint32_t K = (uint32_t)cp.items.size();
-  dbatch_header_kernel<T, DIM><<<(K + 127) / 128, 128, 0, st>>>(tab, K);
-  const auto *map = reinterpret_cast<const unsigned long long *>(dev + cp.map_off);
-  if constexpr (sizeof(T) == 4) {
-    decompress_batch_kernel<T, DIM><<<cp.grid, 32 * DecCfg<T>::warps, dec_smem_bytes<T>(), st>>>(tab, map, cp.work);
-  } else {
-    decompress_batch_kernel<T, DIM, DecCfgF64Fast, kPassFast>
-        <<<cp.grid, 32 * DecCfgF64Fast::warps, dec_smem_bytes_of<DecCfgF64Fast>(), st>>>(tab, map, cp.work);
-    decompress_batch_kernel<T, DIM, DecCfg<T>, kPassGeneral>
-        <<<cp.grid2, 32 * DecCfg<T>::warps, dec_smem_bytes<T>(), st>>>(tab, map, cp.work);
-  }
-}
-
-// Parallel branches on one capturing stream: each begin() goes back to the
-// nodes captured before the first branch, join() makes what follows wait for
-// all of them.  Does nothing when `on` is not set; a failing call invalidates
-// the capture, which its end reports.
-class CaptureBranches {
+// Where a batch's work goes: a stream (one class after another), or a graph,
+// whose classes become parallel branches behind the clearing of the control
+// range.  Each branch beyond the first costs a plan some 45 us when the graph
+// is instantiated and 48 us when it is destroyed, on the host; the graph is
+// built node by node because capturing a stream took another 97 us for that
+// stream's creation and destruction.  A decompress plan of 16 mixed streams
+// that is created, launched once and destroyed: 1,122 us with one branch from
+// a capture and a result copy per stream, 1,237 with branches from a capture,
+// 1,101 so (single-class plans 990 / 847 / 751).
+class Sink {
  public:
-  CaptureBranches(cudaStream_t st, bool on) : st_(st), on_(on) {
-    if (on_) root_ = nodes();
+  explicit Sink(cudaStream_t st) : st_(st) {}
+  explicit Sink(cudaGraph_t graph) : graph_(graph) {}
+
+  // Clears `bytes` (a multiple of 4) at dev; the graph's first node.
+  void clear(uint8_t *dev, uint64_t bytes) {
+    if (!graph_) {
+      cudaMemsetAsync(dev, 0, bytes, st_);
+      return;
+    }
+    cudaMemsetParams m = {};
+    m.dst = dev;
+    m.elementSize = 4;
+    m.width = bytes / 4;
+    m.height = 1;
+    ok_ = ok_ && cudaGraphAddMemsetNode(&root_, graph_, nullptr, 0, &m) == cudaSuccess;
   }
-  void begin() {
-    if (on_) cudaStreamUpdateCaptureDependencies(st_, root_.data(), root_.size(), cudaStreamSetCaptureDependencies);
+  // What follows waits for the clearing alone.
+  void branch() { last_ = root_; }
+
+  template <class... P, class... A>
+  void launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, A... args) {
+    if (!graph_) {
+      kernel<<<grid, threads, smem, st_>>>(args...);
+      return;
+    }
+    std::tuple<P...> values(args...);
+    std::apply(
+        [&](P &...v) {
+          void *ptrs[] = {const_cast<void *>(static_cast<const volatile void *>(&v))...};
+          cudaKernelNodeParams k = {};
+          k.func = reinterpret_cast<void *>(kernel);
+          k.gridDim = grid;
+          k.blockDim = dim3((unsigned)threads);
+          k.sharedMemBytes = (unsigned)smem;
+          k.kernelParams = ptrs;  // copied by the call
+          cudaGraphNode_t node = nullptr;
+          ok_ = ok_ && cudaGraphAddKernelNode(&node, graph_, &last_, 1, &k) == cudaSuccess;
+          last_ = node;
+        },
+        values);
   }
-  void end() {
-    if (!on_) return;
-    const std::vector<cudaGraphNode_t> n = nodes();
-    ends_.insert(ends_.end(), n.begin(), n.end());
-  }
-  void join() {
-    if (on_) cudaStreamUpdateCaptureDependencies(st_, ends_.data(), ends_.size(), cudaStreamSetCaptureDependencies);
-  }
+  bool ok() const { return ok_; }  // graph: every node was added
 
  private:
-  std::vector<cudaGraphNode_t> nodes() const {
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t n = 0;
-    if (cudaStreamGetCaptureInfo(st_, &status, nullptr, nullptr, &deps, &n) != cudaSuccess ||
-        status != cudaStreamCaptureStatusActive)
-      n = 0;
-    return std::vector<cudaGraphNode_t>(deps, deps + n);
-  }
-  cudaStream_t st_;
-  bool on_;
-  std::vector<cudaGraphNode_t> root_, ends_;
+  cudaStream_t st_ = nullptr;
+  cudaGraph_t graph_ = nullptr;
+  cudaGraphNode_t root_ = nullptr, last_ = nullptr;
+  bool ok_ = true;
 };
+
+template <typename T, int DIM>
+void put_class(const gpzb_host::ClassPlan &cp, uint32_t count, uint8_t *dev, uint64_t claim_off, Sink &to) {
+  BItem<T> *tab = reinterpret_cast<BItem<T> *>(dev + cp.table_off);
+  to.branch();
+  if (cp.rel_blocks)
+    to.launch(batch_rel_mapped_kernel<T>, (unsigned)cp.rel_blocks, 256, 0, tab,
+              reinterpret_cast<const unsigned long long *>(dev + cp.rmap_off), count);
+  to.launch(batch_sample_kernel<T>, dim3(128, (unsigned)cp.items.size()), 256, 0, tab);
+  to.launch(compress_batch_kernel<T, DIM>, (unsigned)cp.grid, kEncThreads, sizeof(EncShared), tab,
+            (uint32_t)cp.items.size(), cp.work, reinterpret_cast<unsigned long long *>(dev + claim_off));
+}
+
+template <typename T, int DIM>
+void put_dclass(const gpzb_host::ClassPlan &cp, uint8_t *dev, Sink &to) {
+  DItem<T> *tab = reinterpret_cast<DItem<T> *>(dev + cp.table_off);
+  const uint32_t K = (uint32_t)cp.items.size();
+  to.branch();
+  to.launch(dbatch_header_kernel<T, DIM>, (K + 127) / 128, 128, 0, tab, K);
+  const auto *map = reinterpret_cast<const unsigned long long *>(dev + cp.map_off);
+  if constexpr (sizeof(T) == 4) {
+    to.launch(decompress_batch_kernel<T, DIM>, (unsigned)cp.grid, 32 * DecCfg<T>::warps, dec_smem_bytes<T>(), tab, map,
+              cp.work);
+  } else {
+    to.launch(decompress_batch_kernel<T, DIM, DecCfgF64Fast, kPassFast>, (unsigned)cp.grid, 32 * DecCfgF64Fast::warps,
+              dec_smem_bytes_of<DecCfgF64Fast>(), tab, map, cp.work);
+    to.launch(decompress_batch_kernel<T, DIM, DecCfg<T>, kPassGeneral>, (unsigned)cp.grid2, 32 * DecCfg<T>::warps,
+              dec_smem_bytes<T>(), tab, map, cp.work);
+  }
+}
+
+void put_compress(const gpzb_host::Layout &L, uint8_t *dev, Sink &to) {
+  to.clear(dev, L.zero_bytes);
+  for (int c = 0; c < 4; ++c) {
+    if (L.cls[c].items.empty()) continue;
+    const uint64_t claim = L.claim_off + 8ull * c;
+    switch (c) {
+      case 0: put_class<float, 2>(L.cls[c], L.count, dev, claim, to); break;
+      case 1: put_class<float, 3>(L.cls[c], L.count, dev, claim, to); break;
+      case 2: put_class<double, 2>(L.cls[c], L.count, dev, claim, to); break;
+      default: put_class<double, 3>(L.cls[c], L.count, dev, claim, to); break;
+    }
+  }
+}
+
+void put_decompress(const gpzb_host::Layout &L, uint8_t *dev, Sink &to) {
+  to.clear(dev, L.zero_bytes);
+  for (int c = 0; c < 4; ++c) {
+    if (L.cls[c].items.empty()) continue;
+    switch (c) {
+      case 0: put_dclass<float, 2>(L.cls[c], dev, to); break;
+      case 1: put_dclass<float, 3>(L.cls[c], dev, to); break;
+      case 2: put_dclass<double, 2>(L.cls[c], dev, to); break;
+      default: put_dclass<double, 3>(L.cls[c], dev, to); break;
+    }
+  }
+}
 
 }  // namespace
 
@@ -297,45 +353,20 @@ void decompress_tables(const gpz_dbatch_item *items, const Layout &L, uint8_t *d
   }
 }
 
-void compress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st, bool branches) {
-  cudaMemsetAsync(dev, 0, L.zero_bytes, st);
-  CaptureBranches br(st, branches);
-  for (int c = 0; c < 4; ++c) {
-    if (L.cls[c].items.empty()) continue;
-    const uint64_t claim = L.claim_off + 8ull * c;
-    br.begin();
-    switch (c) {
-      case 0: enqueue_class<float, 2>(L.cls[c], L.count, dev, claim, st); break;
-      case 1: enqueue_class<float, 3>(L.cls[c], L.count, dev, claim, st); break;
-      case 2: enqueue_class<double, 2>(L.cls[c], L.count, dev, claim, st); break;
-      default: enqueue_class<double, 3>(L.cls[c], L.count, dev, claim, st); break;
-    }
-    br.end();
-  }
-  br.join();
+void compress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st) {
+  Sink to(st);
+  put_compress(L, dev, to);
 }
 
-void decompress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st, bool branches) {
-  cudaMemsetAsync(dev, 0, L.zero_bytes, st);
-  CaptureBranches br(st, branches);
-  for (int c = 0; c < 4; ++c) {
-    if (L.cls[c].items.empty()) continue;
-    br.begin();
-    switch (c) {
-      case 0: enqueue_dclass<float, 2>(L.cls[c], dev, st); break;
-      case 1: enqueue_dclass<float, 3>(L.cls[c], dev, st); break;
-      case 2: enqueue_dclass<double, 2>(L.cls[c], dev, st); break;
-      default: enqueue_dclass<double, 3>(L.cls[c], dev, st); break;
-    }
-    br.end();
-  }
-  br.join();
+void decompress_enqueue(const Layout &L, uint8_t *dev, cudaStream_t st) {
+  Sink to(st);
+  put_decompress(L, dev, to);
 }
 
 }  // namespace gpzb_host
 
 // ===========================================================================
-// Plans: the workspace allocated once, the launches captured in a graph.
+// Plans: the workspace allocated once, the launches as a graph.
 // ===========================================================================
 namespace {
 
@@ -351,9 +382,9 @@ struct Plan {
 };
 
 // Allocates the workspace, uploads the table image built by `tables` and
-// captures `enqueue` into the plan's graph.
-template <typename Tables, typename Enq>
-int make_plan(Plan &p, const gpzb_host::Layout &L, Tables tables, Enq enqueue) {
+// builds the plan's graph from what `put` launches.
+template <typename Tables, typename Put>
+int make_plan(Plan &p, const gpzb_host::Layout &L, Tables tables, Put put) {
   p.count = L.count;
   p.bytes = L.bytes;
   if (cudaMalloc(&p.mem, p.bytes) != cudaSuccess) {
@@ -364,17 +395,14 @@ int make_plan(Plan &p, const gpzb_host::Layout &L, Tables tables, Enq enqueue) {
   tables(p.mem, image.data());
   if (cudaMemcpy(p.mem + L.zero_bytes, image.data(), image.size(), cudaMemcpyHostToDevice) != cudaSuccess)
     return GPZ_ECUDA;
-  cudaStream_t s0 = nullptr;
   cudaGraph_t graph = nullptr;
-  bool ok = cudaStreamCreateWithFlags(&s0, cudaStreamNonBlocking) == cudaSuccess &&
-            cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+  bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess;
   if (ok) {
-    enqueue(p.mem, s0);
-    ok = cudaStreamEndCapture(s0, &graph) == cudaSuccess && graph;
+    Sink to(graph);
+    put(L, p.mem, to);
+    ok = to.ok() && cudaGraphInstantiate(&p.exec, graph, 0) == cudaSuccess;
+    cudaGraphDestroy(graph);
   }
-  if (ok) ok = cudaGraphInstantiate(&p.exec, graph, 0) == cudaSuccess;
-  if (graph) cudaGraphDestroy(graph);
-  if (s0) cudaStreamDestroy(s0);
   if (!ok) cudaGetLastError();
   return ok ? GPZ_OK : GPZ_ECUDA;
 }
@@ -420,8 +448,7 @@ int gpz_batch_create(const gpz_batch_item *items, uint32_t count, gpz_batch **ba
   if (!b) return GPZ_ECUDA;
   b->items.assign(items, items + count);
   const int rc = make_plan(
-      b->plan, L, [&](uint8_t *dev, uint8_t *image) { gpzb_host::compress_tables(items, L, dev, image); },
-      [&](uint8_t *dev, cudaStream_t s) { gpzb_host::compress_enqueue(L, dev, s, true); });
+      b->plan, L, [&](uint8_t *dev, uint8_t *image) { gpzb_host::compress_tables(items, L, dev, image); }, put_compress);
   if (rc != GPZ_OK) {
     delete b;
     return rc;
@@ -478,8 +505,7 @@ int gpz_dbatch_create(const gpz_dbatch_item *items, uint32_t count, gpz_dbatch *
   gpz_dbatch *b = new (std::nothrow) gpz_dbatch;
   if (!b) return GPZ_ECUDA;
   const int rc = make_plan(
-      b->plan, L, [&](uint8_t *dev, uint8_t *image) { gpzb_host::decompress_tables(items, L, dev, image); },
-      [&](uint8_t *dev, cudaStream_t s) { gpzb_host::decompress_enqueue(L, dev, s, true); });
+      b->plan, L, [&](uint8_t *dev, uint8_t *image) { gpzb_host::decompress_tables(items, L, dev, image); }, put_decompress);
   if (rc != GPZ_OK) {
     delete b;
     return rc;

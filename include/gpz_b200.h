@@ -275,7 +275,7 @@ int gpz_stream_size(const void *d_stream, uint64_t cap, uint64_t *bytes, void *s
  * A batch is a plan bound to the buffers named in its items (like an FFT
  * plan): gpz_batch_create validates the items, allocates the batch's device
  * memory (descriptors, work maps, control blocks and look-back records per
- * snapshot) and captures the graph; gpz_batch_launch replays it on a stream
+ * snapshot) and builds the graph; gpz_batch_launch runs it on a stream
  * (the inputs may change between launches, the pointers and sizes may not);
  * gpz_batch_results synchronises the stream and reads every snapshot's result.
  * Launches of one batch must not overlap on the GPU. */
