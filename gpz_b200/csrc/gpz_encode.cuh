@@ -360,7 +360,10 @@ static __device__ __noinline__ void warp_sort_small(uint32_t *a, uint32_t n, int
 // ids of two passes; 3D points on 40 sites 366 -> 296 us.
 static __device__ __noinline__ void cta_sort(uint32_t *H, uint32_t *S) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  __syncthreads();  // the ids by rank are in place
   uint32_t v[kEncPer];
+#pragma unroll
+  for (int e = 0; e < kEncPer; ++e) v[e] = (S[rx(kEncPer * t + e)] << 10) | (uint32_t)(kEncPer * t + e);
   auto get = [](const uint32_t *buf, int from, uint32_t (&o)[kEncPer]) {
     const uint4 a = ld4(buf + 4 * from), b = ld4(buf + 4 * (kEncThreads + from));
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
@@ -383,9 +386,6 @@ static __device__ __noinline__ void cta_sort(uint32_t *H, uint32_t *S) {
 #pragma unroll
     for (int j = 16 * kEncPer; j > 0; j >>= 1) exchange<kEncPer>(v, lane, 0, j);
   };
-  __syncthreads();  // the ids by rank are in place
-#pragma unroll
-  for (int e = 0; e < kEncPer; ++e) v[e] = (S[rx(kEncPer * t + e)] << 10) | (uint32_t)(kEncPer * t + e);
   warp_sort<kEncPer>(v, lane);
   cross(H, t ^ 63, true, (warp & 1) != 0);    // i with i ^ 511
   finish();
@@ -415,6 +415,40 @@ struct Points {
   }
   __host__ __device__ constexpr static uint32_t rank_step(int e) { return 32u * (e % kVec) + 4u * kVec * (e / kVec); }
 };
+
+// First position that warp `warp` orders: its own 256 and kEncHalo more on
+// either side (all on one side at the chunk's ends).
+__host__ __device__ constexpr uint32_t ord_window(int warp) {
+  return warp == 0 ? 0u : (warp == kEncWarps - 1 ? kChunk - 32u * kEncOrd : 256u * warp - kEncHalo);
+}
+
+// Odd-even transposition over a lane's kEncOrd positions: the even (h = 0) or
+// odd (h = 1) pairs.  cut[j] is all ones where positions j and j + 1 are not to
+// be exchanged (wide form; the narrow one's neighbours of different buckets are
+// in order already).
+template <bool kNarrow>
+__host__ __device__ __forceinline__ void order_pairs(uint32_t (&k)[kEncOrd], const uint32_t (&cut)[kEncOrd], int h) {
+#pragma unroll
+  for (int j = h; j + 1 < kEncOrd; j += 2) {
+    const uint32_t x = k[j], y = k[j + 1];
+    k[j] = min(x, kNarrow ? y : y | cut[j]);
+    k[j + 1] = max(kNarrow ? x : x & ~cut[j], y);
+  }
+}
+
+// The pairs across lanes: nx is the next lane's first value, pv the previous
+// lane's last, pcut the previous lane's last cut.
+template <bool kNarrow>
+__host__ __device__ __forceinline__ void order_across(uint32_t (&k)[kEncOrd], const uint32_t (&cut)[kEncOrd], uint32_t nx,
+                                                      uint32_t pv, uint32_t pcut, int lane) {
+  if (kNarrow) {
+    if (lane < 31) k[kEncOrd - 1] = min(k[kEncOrd - 1], nx);
+    if (lane > 0) k[0] = max(k[0], pv);
+  } else {
+    k[kEncOrd - 1] = min(k[kEncOrd - 1], nx | cut[kEncOrd - 1]);
+    k[0] = max(k[0], pv & ~pcut);
+  }
+}
 
 // Ranks a full chunk's points through buckets over their id range.
 //  * kNarrow (ids below 2^22): 1024 buckets that split the range evenly
@@ -531,26 +565,18 @@ __device__ __forceinline__ bool rank_buckets(RankShared &sm, uint32_t *H, uint32
   // in the order even pairs, across lanes, odd pairs, across lanes: ceil(n / 2)
   // rounds order a bucket of n points wherever it lies.
   uint32_t k9[kEncOrd];
-  const uint32_t w0 = warp == 0 ? 0u : (warp == kEncWarps - 1 ? kChunk - 32u * kEncOrd : 256u * warp - kEncHalo);
-  const uint32_t p0 = w0 + kEncOrd * lane, o0 = p0 - 256u * warp;
+  const uint32_t p0 = ord_window(warp) + kEncOrd * lane, o0 = p0 - 256u * warp;
 #pragma unroll
   for (int j = 0; j < kEncOrd; ++j) k9[j] = S[p0 + j];
   const uint32_t rounds = (largest + 1u) >> 1;
   if (kNarrow) {
-    // neighbours of different buckets are in order already
 #pragma unroll 1
     for (uint32_t it = 0; it < rounds; ++it) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int j = h; j + 1 < kEncOrd; j += 2) {
-          const uint32_t x = k9[j], y = k9[j + 1];
-          k9[j] = min(x, y);
-          k9[j + 1] = max(x, y);
-        }
+        order_pairs<true>(k9, k9, h);
         const uint32_t nx = __shfl_down_sync(FULL, k9[0], 1), pv = __shfl_up_sync(FULL, k9[kEncOrd - 1], 1);
-        if (lane < 31) k9[kEncOrd - 1] = min(k9[kEncOrd - 1], nx);
-        if (lane > 0) k9[0] = max(k9[0], pv);
+        order_across<true>(k9, k9, nx, pv, 0u, lane);
       }
     }
 #pragma unroll
@@ -574,15 +600,9 @@ __device__ __forceinline__ bool rank_buckets(RankShared &sm, uint32_t *H, uint32
     for (uint32_t it = 0; it < rounds; ++it) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int j = h; j + 1 < kEncOrd; j += 2) {
-          const uint32_t x = k9[j], y = k9[j + 1];
-          k9[j] = min(x, y | cut[j]);
-          k9[j + 1] = max(x & ~cut[j], y);
-        }
+        order_pairs<false>(k9, cut, h);
         const uint32_t nx = __shfl_down_sync(FULL, k9[0], 1), pv = __shfl_up_sync(FULL, k9[kEncOrd - 1], 1);
-        k9[kEncOrd - 1] = min(k9[kEncOrd - 1], nx | cut[kEncOrd - 1]);
-        k9[0] = max(k9[0], pv & ~pcut);
+        order_across<false>(k9, cut, nx, pv, pcut, lane);
       }
     }
 #pragma unroll
