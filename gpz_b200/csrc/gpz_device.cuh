@@ -171,7 +171,6 @@ __device__ __forceinline__ void warp_minmax(const double (&v)[N], double &mn, do
 }
 
 __device__ __forceinline__ uint32_t bitlen(uint32_t v) { return 32u - (uint32_t)__clz(v); }
-__device__ __forceinline__ uint32_t bitlen64(unsigned long long v) { return 64u - (uint32_t)__clzll(v); }
 
 // Section sizes (src/cudaWarpCompress.cu:324-328; Double :325-329).
 __host__ __device__ __forceinline__ uint32_t section_bytes(uint32_t U, uint32_t nbits, uint32_t pad) {

@@ -141,48 +141,33 @@ __device__ __forceinline__ void put_plane_bytes(uint8_t *d, int room, uint32_t w
   if (room > 3) d[3] = (uint8_t)w;
 }
 
-// Bit planes b0..b0+N-1 (those below nb; N = 8 or 16, b0 a multiple of 8) of a
-// 1024-element array (swizzled rows) by one warp: lane l takes elements
-// 32l..32l+31, gathers the N bits of each and turns them into plane words.
+// Bit planes b0..b0+7 (those below nb; b0 a multiple of 8) of a 1024-element
+// array (swizzled rows) by one warp: lane l takes elements 32l..32l+31, gathers
+// the eight bits of each and turns them into plane words.
 // Planes go MSB plane first to byte pos0 of the staged payload: byte planes of
 // bpp bytes (bpp != 0) or planes of 32 words.
-template <int N>
 __device__ __forceinline__ void plane_job(const uint32_t *arr, uint8_t *stage, uint32_t pos0, uint32_t nb, uint32_t b0,
                                           uint32_t bpp, int lane) {
-  uint32_t w[N];
+  uint32_t w[8];
   const uint32_t k = b0 >> 3;
-  if constexpr (N == 8) {
-    const uint32_t s0 = k | ((4u + k) << 4);  // byte k of both sources
+  const uint32_t s0 = k | ((4u + k) << 4);  // byte k of both sources
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      // quads h, h+2, h+4, h+6 of the row: elements 4h.. (+0, +8, +16, +24)
-      const uint4 q0 = ld4(arr + qoff(lane, h)), q1 = ld4(arr + qoff(lane, h + 2));
-      const uint4 q2 = ld4(arr + qoff(lane, h + 4)), q3 = ld4(arr + qoff(lane, h + 6));
-      w[4 * h + 0] = prmt(prmt(q0.x, q1.x, s0), prmt(q2.x, q3.x, s0), 0x5410);
-      w[4 * h + 1] = prmt(prmt(q0.y, q1.y, s0), prmt(q2.y, q3.y, s0), 0x5410);
-      w[4 * h + 2] = prmt(prmt(q0.z, q1.z, s0), prmt(q2.z, q3.z, s0), 0x5410);
-      w[4 * h + 3] = prmt(prmt(q0.w, q1.w, s0), prmt(q2.w, q3.w, s0), 0x5410);
-    }
-  } else {
-    const uint32_t s0 = k ? 0x7632u : 0x5410u;  // half k/2 of both sources
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      // quads h, h+4: elements 4h.. and 16 + 4h..
-      const uint4 q0 = ld4(arr + qoff(lane, h)), q1 = ld4(arr + qoff(lane, h + 4));
-      w[4 * h + 0] = prmt(q0.x, q1.x, s0);
-      w[4 * h + 1] = prmt(q0.y, q1.y, s0);
-      w[4 * h + 2] = prmt(q0.z, q1.z, s0);
-      w[4 * h + 3] = prmt(q0.w, q1.w, s0);
-    }
-    byte_stage<16>(w);
+  for (int h = 0; h < 2; ++h) {
+    // quads h, h+2, h+4, h+6 of the row: elements 4h.. (+0, +8, +16, +24)
+    const uint4 q0 = ld4(arr + qoff(lane, h)), q1 = ld4(arr + qoff(lane, h + 2));
+    const uint4 q2 = ld4(arr + qoff(lane, h + 4)), q3 = ld4(arr + qoff(lane, h + 6));
+    w[4 * h + 0] = prmt(prmt(q0.x, q1.x, s0), prmt(q2.x, q3.x, s0), 0x5410);
+    w[4 * h + 1] = prmt(prmt(q0.y, q1.y, s0), prmt(q2.y, q3.y, s0), 0x5410);
+    w[4 * h + 2] = prmt(prmt(q0.z, q1.z, s0), prmt(q2.z, q3.z, s0), 0x5410);
+    w[4 * h + 3] = prmt(prmt(q0.w, q1.w, s0), prmt(q2.w, q3.w, s0), 0x5410);
   }
-  low_stages<N>(w);
-  const uint32_t left = nb - b0;  // planes of this job (all N, or the top ones)
+  low_stages<8>(w);
+  const uint32_t left = nb - b0;  // planes of this job (all 8, or the top ones)
   if (bpp) {
     const int room = (int)bpp - 4 * lane;
     uint8_t *d = stage + pos0 + (left - 1u) * bpp + 4u * lane;
 #pragma unroll
-    for (int b = 0; b < N; ++b) {
+    for (int b = 0; b < 8; ++b) {
       if ((uint32_t)b >= left) break;
       put_plane_bytes(d, room, w[b]);
       d -= bpp;
@@ -190,7 +175,7 @@ __device__ __forceinline__ void plane_job(const uint32_t *arr, uint8_t *stage, u
   } else {
     uint32_t *d = reinterpret_cast<uint32_t *>(stage + pos0) + 32u * (left - 1u) + lane;
 #pragma unroll
-    for (int b = 0; b < N; ++b) {
+    for (int b = 0; b < 8; ++b) {
       if ((uint32_t)b >= left) break;
       d[-32 * b] = w[b];
     }
@@ -1097,9 +1082,9 @@ __device__ __forceinline__ uint32_t encode_chunk(const CArgs<T> &a, unsigned lon
     // jobs of eight planes, the longest first
     const uint32_t nd = (dbits + 7u) >> 3, nr = (rbits + 7u) >> 3, nc = (cbits + 7u) >> 3;
     for (uint32_t j = warp; j < nd + nr + nc; j += kEncWarps) {
-      if (j - nd < nr) plane_job<8>(sm.Q, stage, db + cb, rbits, 8u * (j - nd), 0u, lane);
-      else if (j < nd) plane_job<8>(H, stage, 0u, dbits, 8u * j, bpp, lane);
-      else plane_job<8>(sm.R, stage, db, cbits, 8u * (j - nd - nr), bpp, lane);
+      if (j - nd < nr) plane_job(sm.Q, stage, db + cb, rbits, 8u * (j - nd), 0u, lane);
+      else if (j < nd) plane_job(H, stage, 0u, dbits, 8u * j, bpp, lane);
+      else plane_job(sm.R, stage, db, cbits, 8u * (j - nd - nr), bpp, lane);
     }
   }
   if (warp == kEncWarps - 1) {
