@@ -211,7 +211,7 @@ __device__ __forceinline__ uint32_t warp_inc_scan(uint32_t v, int lane) {
 // number.  ceil(bits / 9) passes.
 // byr: ids by rank (rx); cnt: 4 KB of counters; perm: two permutations of
 // 1024 ranks.  Begins and ends with a barrier; returns the sorted ranks.
-static __device__ __noinline__ const uint16_t *radix_rank(const uint32_t *byr, uint32_t *scr, uint16_t *perm,
+__device__ __forceinline__ const uint16_t *radix_rank(const uint32_t *byr, uint32_t *scr, uint16_t *perm,
                                                           uint32_t *tot, uint32_t idbits) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -343,7 +343,7 @@ static __device__ __noinline__ void warp_sort_small(uint32_t *a, uint32_t n, int
 // passes at these ids: 20M float points, half of them in one place, 396 -> 296
 // us in 2D (19-bit ids) and 419 -> 309 us in 3D (21 bits), 292 -> 280 us with
 // ids of two passes; 3D points on 40 sites 366 -> 296 us.
-static __device__ __noinline__ void cta_sort(uint32_t *H, uint32_t *S) {
+__device__ __forceinline__ void cta_sort(uint32_t *H, uint32_t *S) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   __syncthreads();  // the ids by rank are in place
   uint32_t v[kEncPer];
@@ -381,6 +381,17 @@ static __device__ __noinline__ void cta_sort(uint32_t *H, uint32_t *S) {
   *reinterpret_cast<uint4 *>(H + 8 * t) = make_uint4(v[0], v[1], v[2], v[3]);
   *reinterpret_cast<uint4 *>(H + 8 * t + 4) = make_uint4(v[4], v[5], v[6], v[7]);
   __syncthreads();
+}
+
+// Ranks a chunk that the buckets do not, from the ids by rank in S: by the
+// CTA's network (`network`; nullptr, the sorted composites in H) or by the radix
+// sort (the sorted ranks).  One call for both: with two, the batch kernels spilt
+// more (7.75 -> 7.84 ms for the bench's 256 snapshots).
+static __device__ __noinline__ const uint16_t *rank_rest(uint32_t *H, uint32_t *S, uint16_t *perm, uint32_t *tot,
+                                                         uint32_t idbits, bool network) {
+  if (!network) return radix_rank(S, H, perm, tot, idbits);
+  cta_sort(H, S);
+  return nullptr;
 }
 
 // A chunk's points in registers, one 16-byte load (kVec points) at a time:
@@ -701,11 +712,9 @@ __device__ __forceinline__ int rank_chunk(RankShared &sm, uint32_t *H, uint32_t 
     }
 #pragma unroll
     for (int e = 0; e < kEncPer; ++e) S[rx(rbase + Points<T>::rank_step(e))] = key[e];
-    if (full && narrow && bound >= kEncOnePass) {
-      cta_sort(H, S);
-      return 1;
-    }
-    ranks = radix_rank(S, H, reinterpret_cast<uint16_t *>(sm.Q), sm.tot, bitlen(bound + (full ? 0u : 1u)));
+    ranks = rank_rest(H, S, reinterpret_cast<uint16_t *>(sm.Q), sm.tot, bitlen(bound + (full ? 0u : 1u)),
+                      full && narrow && bound >= kEncOnePass);
+    if (ranks == nullptr) how = 1;
   }
   return how;
 }
