@@ -142,11 +142,9 @@ __global__ void __launch_bounds__(kEncThreads, kEncCtas)
     const T inv = is64 ? (T)__ddiv_rn(1.0, __dmul_rn(2.0, (double)eb)) : (T)__fdiv_rn(1.0f, __fmul_rn(2.0f, (float)eb));
     const uint32_t slot = encode_chunk<T, DIM>(a, c, sm, par, seg, eb, inv, bs.parked, pk, rank_skip, declined, claim_next,
                                                [&]() { fetch(par ^ 1); });
-    // the next look-up is the first warp's, before a barrier
-    if (warp == 0) {
-      copy_args(bs.parked[slot], a, lane);
-      __syncwarp();
-    }
+    // every look-up of this payload comes behind the next chunk's first barrier
+    // or the flush's
+    if (warp == 0) copy_args(bs.parked[slot], a, lane);
     par ^= 1;
   }
   flush_parked<T>(bs.parked, sm, pk, lane, warp);

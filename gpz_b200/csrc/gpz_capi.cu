@@ -3,9 +3,10 @@
 // Host orchestration replacing CudaWarpCompress::compressImpl /
 // decompressImpl (reference src/cudaWarpCompress.cu:1573-1856 and the double
 // twin): no allocation, no host synchronisation and no small memcpys inside
-// the call -- one memset of the scratch control block, the sampling kernel
-// that resolves the segment size on the device, and one persistent
-// compress kernel that writes the finished stream.
+// the call -- one memset of the scratch control block and look-back records,
+// the sampling kernel that resolves the segment size on the device (up to
+// 16,384 points one block does both), and one persistent compress kernel that
+// writes the finished stream.
 
 #include <algorithm>
 #include <cstdio>
@@ -559,8 +560,8 @@ int gpz_compress_noalloc(const gpz_params *params, const void *d_x, const void *
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// Check of the bounded wait of the placement look-back: group 1 waits on a
-// group 0 that never publishes its size (its field of the record stays zero, as if
+// Check of the bounded wait of the placement look-back: chunk 1 waits on a
+// chunk 0 that never publishes its size (its field of the record stays zero, as if
 // the CTA holding it had stopped), so the wait runs out after `polls` polls.
 // ---------------------------------------------------------------------------
 namespace {

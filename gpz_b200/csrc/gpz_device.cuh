@@ -2,10 +2,11 @@
 //
 // Layout and arithmetic follow the GPZ reference format (path:line citations
 // refer to the reference project); the parallel decomposition is this
-// library's own: one warp per 1024-point chunk in persistent grids, register
-// sorting networks for the stable order by block id, in-register bit
-// transposes for the bit planes, and a single-pass decoupled look-back scan
-// that places each group's payloads directly in the output stream.
+// library's own: persistent grids, a CTA of four warps per 1024-point chunk to
+// compress and one warp per chunk to decompress, bucket, network or radix
+// ranking for the stable order by block id, in-register bit transposes for the
+// bit planes, and a single-pass decoupled look-back over the chunks' sizes that
+// gives every parked payload its place in the output stream.
 #pragma once
 
 #include <cfloat>
@@ -279,6 +280,9 @@ __host__ __device__ __forceinline__ void transpose32(uint32_t (&a)[32]) {
   low_stages<32>(a);
 }
 
+// The next three, pair_value, quad_value and to_msb_bytes are used by the CPU
+// check of the transposes alone (tests/host/transpose_check.cu).
+//
 // Planes 0..15 only (values that need <= 16 bits): a[b] = plane b, b < 16.
 __host__ __device__ __forceinline__ void transpose_lo16(uint32_t (&a)[32]) {
 #pragma unroll

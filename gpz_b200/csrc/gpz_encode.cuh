@@ -338,11 +338,12 @@ static __device__ __noinline__ void warp_sort_small(uint32_t *a, uint32_t n, int
 // through S and H in turn.  S: ids by rank (rx); H: the sorted composites.
 // Begins and ends with a barrier.
 //
-// Bound by instruction issue: 700 instructions a warp and five barriers, on any
-// input.  The radix sort takes 350 and six barriers a pass, and two or three
-// passes at these ids: 20M float points, half of them in one place, 396 -> 296
-// us in 2D (19-bit ids) and 419 -> 309 us in 3D (21 bits), 292 -> 280 us with
-// ids of two passes; 3D points on 40 sites 366 -> 296 us.
+// Bound by instruction issue, the same on any input, with six barriers.  The
+// radix sort has five a pass, two or three passes at these ids, and its match.any
+// takes the longer the more digits differ.  20M float points, half of them in one
+// place: 396 -> 296 us in 2D (19-bit ids; 10.2 -> 8.8 K warp instructions and 3.1
+// -> 2.4 K shared wavefronts a chunk), 419 -> 309 us in 3D (21 bits), 292 -> 280
+// us with ids of two passes; 3D points on 40 sites 366 -> 296 us.
 __device__ __forceinline__ void cta_sort(uint32_t *H, uint32_t *S) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   __syncthreads();  // the ids by rank are in place
@@ -461,9 +462,16 @@ __host__ __device__ __forceinline__ void order_across(uint32_t (&k)[kEncOrd], co
 //
 // 32M clustered points with a few percent of them in one cluster: 0.85 ms when
 // any bucket of 16 points sent the chunk to the radix sort (three passes at
-// these id ranges), 0.41 ms so, 0.51 ms in the one-warp form.  Points in many
-// crowded buckets (ordered snapshots) are cheaper in the radix sort: hence the
-// second limit.
+// these id ranges), 0.41 ms so, 0.51 ms in the one-warp form.
+//
+// The limits, by 20M float points of which a share lies in one place (2D, us;
+// with kEncCrowd 128 / 192 / 256): 15 % 288 / 262 / 261, 20 % 282 / 310 / 263,
+// 25 % 285 / 298 / 342, 30 % 289 / 297 / 307, 50 % 294 / 294 / 296.  One warp
+// sorts such a bucket while three wait, so the limit's worth lies below it, and
+// chunks on both sides of it in turn are the worst case.  Many crowded buckets
+// (with kEncCrowdPoints 256 / 512 / 1024): an integer grid 269 / 269 / 346, 3D
+// points on 40 sites 296 / 296 / 384.  kEncBucketBackoff 8 / 16: 25 % 342 / 329,
+// 90 % 320 / 317, the others within 1 %.
 template <typename T, bool kNarrow>
 __device__ __forceinline__ bool rank_buckets(RankShared &sm, uint32_t *H, uint32_t *S, const uint32_t (&key)[kEncPer],
                                              uint32_t bound, int t, int lane, int warp) {

@@ -218,7 +218,7 @@ __host__ __device__ inline T strict_bound(T eb, double max_abs, double max_range
 // inverted; NaNs ignored, -0 below +0).
 //
 // A pure read, bound by HBM: every thread keeps kFoldUnroll 16-byte loads in
-// flight (64 bytes; 8 blocks of 256 threads per SM hold 128 KB in flight, four
+// flight (64 bytes; 6 blocks of 256 threads per SM hold 96 KB in flight, 2.7
 // times what 6.5 TB/s needs at ~800 ns), and a float axis is folded with
 // three-input min / max, half an instruction per value each.  rel_to_abs on
 // 143,735,721 float 3D points: 2.33 ms with one scalar load per thread, axis
